@@ -453,6 +453,16 @@ typedef struct srt_bgemm_desc { /* D[z][m][n] = alpha * sum_k A[z][m][k] B[z][n]
   int k_causal; /* 1: A is zero for k > m, 2: A is zero for k < m */
 } srt_bgemm_desc;
 int srt_bgemm(const srt_bgemm_desc* d, const void* A, const void* B, void* D, void* stream);
+/* Attention with 64-channel heads over the heads of [B*S][ld] matrices (head h at column 64 h; K and V have Hkv heads, each
+ * read by H / Hkv query heads). rows: three arrays of [B*H][S rounded up to 128] floats, written by forward (where it may
+ * be null) and read by backward. Backward is causal; dK and dV come per query head with strides (position, head, batch) =
+ * (ld_dkv, dkv_s1, dkv_s2). */
+typedef struct srt_attention_shape { int B, S, H, Hkv, D; } srt_attention_shape;
+int srt_attention_fwd(const srt_attention_shape* a, const void* Q, const void* K, const void* V, long long ld_qkv, void* O,
+                      long long ld_o, float* rows, float scale, int causal, void* stream);
+int srt_attention_bwd_causal(const srt_attention_shape* a, const void* Q, const void* K, const void* V, long long ld_qkv,
+                             const void* dO, long long ld_o, float* rows, void* dQ, long long ld_dq, void* dK, void* dV,
+                             long long ld_dkv, long long dkv_s1, long long dkv_s2, float scale, void* stream);
 int srt_layernorm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd,
                       int64_t rows, int C, float eps, void* stream);
 size_t srt_layernorm_bwd_scratch_bytes(int C);

@@ -405,6 +405,18 @@ int srt_bgemm(const srt_bgemm_desc* d, const void* A, const void* B, void* D, vo
                  d->ldd, d->d_s1, d->d_s2, d->alpha, d->causal, d->k_causal};
   return bgemm_bf16(g, A, B, D, (cudaStream_t)stream);
 }
+int srt_attention_fwd(const srt_attention_shape* a, const void* Q, const void* K, const void* V, long long ld_qkv, void* O,
+                      long long ld_o, float* rows, float scale, int causal, void* stream) {
+  SRT_REQUIRE(a && Q && K && V && O, "attention_fwd: null argument");
+  return attention_fwd({a->B, a->S, a->H, a->Hkv, a->D}, Q, K, V, ld_qkv, O, ld_o, rows, scale, causal, (cudaStream_t)stream);
+}
+int srt_attention_bwd_causal(const srt_attention_shape* a, const void* Q, const void* K, const void* V, long long ld_qkv,
+                             const void* dO, long long ld_o, float* rows, void* dQ, long long ld_dq, void* dK, void* dV,
+                             long long ld_dkv, long long dkv_s1, long long dkv_s2, float scale, void* stream) {
+  SRT_REQUIRE(a && Q && K && V && dO && rows && dQ && dK && dV, "attention_bwd: null argument");
+  return attention_bwd_causal({a->B, a->S, a->H, a->Hkv, a->D}, Q, K, V, ld_qkv, dO, ld_o, rows, dQ, ld_dq, dK, dV, ld_dkv,
+                              dkv_s1, dkv_s2, scale, (cudaStream_t)stream);
+}
 int srt_layernorm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd,
                       int64_t rows, int C, float eps, void* stream) {
   SRT_REQUIRE(x && gamma && beta && y && mean && rstd, "layernorm_fwd: null argument");

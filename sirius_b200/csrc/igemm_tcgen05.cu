@@ -1535,6 +1535,11 @@ int launch_bgemm(const BgemmParams& p, const CUtensorMap& ta, const CUtensorMap&
 
 }  // namespace
 
+int tmap_batched_bf16(CUtensorMap* tm, const void* base, uint64_t kdim, uint64_t rows, uint64_t z1, uint64_t z2, uint64_t ld,
+                      uint64_t s1, uint64_t s2, uint32_t box_rows) {
+  return make_tmap_4d(tm, base, kdim, rows, z1, z2, ld, s1, s2, box_rows);
+}
+
 int bgemm_bf16(const BgemmDesc& d, const void* A, const void* B, void* D, cudaStream_t st) {
   SRT_REQUIRE(d.M > 0 && d.N > 0 && d.K > 0 && d.Z1 > 0 && d.Z2 > 0, "bgemm: empty problem");
   SRT_REQUIRE(d.K % 8 == 0 && d.N % 8 == 0 && d.ldd % 8 == 0 && d.d_s1 % 8 == 0 && d.d_s2 % 8 == 0 &&

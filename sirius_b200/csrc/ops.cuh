@@ -97,6 +97,21 @@ struct BgemmDesc {
 };
 int bgemm_bf16(const BgemmDesc& d, const void* A, const void* B, void* D, cudaStream_t st);
 
+// Attention with 64-channel heads, without the score matrix in memory (attention_tcgen05.cu). Q, K, V are the heads of
+// [B*S][ld] matrices (head h at column 64 h; K and V have Hkv heads, each shared by H / Hkv query heads), O and dO
+// likewise. rows: three arrays of [B*H][attention_s_pad(S)] floats, the maximum and inverse sum of every row (written by
+// forward, optional there) and the row term of the backward pass. dK and dV are written per query head with strides
+// (position, head, batch) = (ld_dkv, dkv_s1, dkv_s2).
+struct AttentionShape { int B, S, H, Hkv, D; };
+inline bool attention_supported(int D) { return D == 64; }
+int attention_s_pad(int S);
+inline size_t attention_rows_floats(int B, int S, int H) { return (size_t)3 * B * H * attention_s_pad(S); }
+int attention_fwd(const AttentionShape& a, const void* Q, const void* K, const void* V, long long ld_qkv, void* O, long long ld_o,
+                  float* rows, float scale, int causal, cudaStream_t st);
+int attention_bwd_causal(const AttentionShape& a, const void* Q, const void* K, const void* V, long long ld_qkv, const void* dO,
+                         long long ld_o, float* rows, void* dQ, long long ld_dq, void* dK, void* dV, long long ld_dkv,
+                         long long dkv_s1, long long dkv_s2, float scale, cudaStream_t st);
+
 int layernorm_fwd(const void* x, const float* gamma, const float* beta, void* y, float* mean, float* rstd,
                   int64_t rows, int C, float eps, cudaStream_t st);
 // RMSNorm: y = x * rsqrt(mean(x^2) + eps) * gamma. Backward through layernorm_bwd with rms = 1 (mean holds zeros).

@@ -160,9 +160,11 @@ int Bert::alloc_activations() {
   int rc;
   auto act = [&](__nv_bfloat16** p, size_t elems) { return aalloc((void**)p, elems * 2); };
   if ((rc = act(&emb, T * C)) || (rc = act(&xa, T * C)) || (rc = act(&xb, T * C)) || (rc = act(&qkv, T * 3 * C)) ||
-      (rc = act(&Pm, BH * S * S)) || (rc = act(&vt, T * C)) || (rc = act(&att, T * C)) || (rc = act(&t1, T * C)) ||
+      (rc = act(&att, T * C)) || (rc = act(&t1, T * C)) ||
       (rc = act(&sa, T * C)) || (rc = act(&h1, T * F)) || (rc = act(&g1, T * F)))
     return rc;
+  // head sizes other than 64 go through the score matrix
+  if (!attention_supported(D) && ((rc = act(&Pm, BH * S * S)) || (rc = act(&vt, T * C)))) return rc;
   if ((rc = aalloc((void**)&mean, T * 4)) || (rc = aalloc((void**)&rstd, T * 4))) return rc;
   return SRT_OK;
 }
@@ -177,16 +179,20 @@ int Bert::forward(int B) {
   __nv_bfloat16 *x = xa, *nxt = xb;
   for (Layer& y : layers) {
     if ((rc = linear(y.wq, y.bq, C, 3 * C, x, qkv, nullptr, T))) return rc;
-    // scores = Q K^T / sqrt(D) per (batch, head), all S x S entries
-    BgemmDesc q = {S, S, D, H, B, 3LL * C, D, (long long)S * 3 * C, 3LL * C, D, (long long)S * 3 * C,
-                   S, (long long)S * S, (long long)H * S * S, scale, 0, 0};
-    if ((rc = bgemm_bf16(q, qkv, qkv + C, Pm, stream))) return rc;
-    if ((rc = softmax_rows_fwd(Pm, (int64_t)B * H * S, S, stream))) return rc;
-    // context = P V: the B operand is V^T per head, [B][H][D][S]
-    if ((rc = batched_transpose(qkv + 2 * C, vt, S, D, 3LL * C, D, (long long)S * 3 * C, H, B, stream))) return rc;
-    BgemmDesc o = {S, D, S, H, B, S, (long long)S * S, (long long)H * S * S, S, (long long)D * S, (long long)H * D * S,
-                   C, D, (long long)S * C, 1.f, 0, 0};
-    if ((rc = bgemm_bf16(o, Pm, vt, att, stream))) return rc;
+    if (attention_supported(D)) {
+      if ((rc = attention_fwd({B, S, H, H, D}, qkv, qkv + C, qkv + 2 * C, 3LL * C, att, C, nullptr, scale, 0, stream))) return rc;
+    } else {
+      // scores = Q K^T / sqrt(D) per (batch, head), all S x S entries
+      BgemmDesc q = {S, S, D, H, B, 3LL * C, D, (long long)S * 3 * C, 3LL * C, D, (long long)S * 3 * C,
+                     S, (long long)S * S, (long long)H * S * S, scale, 0, 0};
+      if ((rc = bgemm_bf16(q, qkv, qkv + C, Pm, stream))) return rc;
+      if ((rc = softmax_rows_fwd(Pm, (int64_t)B * H * S, S, stream))) return rc;
+      // context = P V: the B operand is V^T per head, [B][H][D][S]
+      if ((rc = batched_transpose(qkv + 2 * C, vt, S, D, 3LL * C, D, (long long)S * 3 * C, H, B, stream))) return rc;
+      BgemmDesc o = {S, D, S, H, B, S, (long long)S * S, (long long)H * S * S, S, (long long)D * S, (long long)H * D * S,
+                     C, D, (long long)S * C, 1.f, 0, 0};
+      if ((rc = bgemm_bf16(o, Pm, vt, att, stream))) return rc;
+    }
     if ((rc = linear(y.wo, y.bo, C, C, att, t1, x, T))) return rc;                                   // + residual
     if ((rc = layernorm_fwd(t1, pf(y.ln1_g), pf(y.ln1_b), sa, mean, rstd, T, C, cfg.ln_eps, stream))) return rc;
     if ((rc = linear(y.w1, y.b1, C, F, sa, h1, nullptr, T))) return rc;

@@ -5,9 +5,9 @@
 //
 // Data layout: activations are [tokens][features] bf16 rows (tokens = batch * seq); every linear layer is
 // a 1x1 convolution over that matrix and runs on the tcgen05 implicit-GEMM kernels (bias and residual
-// add in the epilogue); attention products are batched tcgen05 GEMMs that address the heads inside the
-// fused [tokens][3*d] projection through 4-D tensor maps; parameters, gradients and both AdamW moments are
-// flat fp32 buffers with a bf16 working copy. Linear weights are stored [out][in] (the reference's Conv1D
+// add in the epilogue); attention addresses the heads inside the fused [tokens][3*d] projection through 4-D
+// tensor maps (fused kernels for 64-channel heads, batched tcgen05 GEMMs for other sizes); parameters, gradients
+// and both AdamW moments are flat fp32 buffers with a bf16 working copy. Linear weights are stored [out][in] (the reference's Conv1D
 // keeps [in][out]; set/get transpose).
 #include <string.h>
 
@@ -49,6 +49,7 @@ struct Gpt2 {
     // saved activations
     __nv_bfloat16 *ln1o, *qkv_o, *Pm, *att, *x2, *ln2o, *h, *g, *xout;
     float *ln1_mean, *ln1_rstd, *ln2_mean, *ln2_rstd;
+    float* rows;  // maximum, inverse sum and backward term of the score rows (64-channel heads, which keep no score matrix)
   };
   std::vector<Layer> layers;
   int wte, wpe, lnf_g, lnf_b;
@@ -198,6 +199,8 @@ struct Gpt2 {
 
   int build();
   int refresh();
+  int attention_forward(Layer& y, int B, float scale);
+  int attention_backward(Layer& y, int B, float scale);
   int forward(int B);
   int backward(int B, int global_batch);
   srt_conv_desc lin_desc(int64_t T, int in, int out) const { return {(int)T, 1, 1, in, out, 1, 1, 1, 0, 1, 1}; }
@@ -303,11 +306,13 @@ int Gpt2::alloc_activations(int B) {
   int rc = free_activation_blocks();
   if (rc) return rc;
   const size_t T = (size_t)B * S, BH = (size_t)B * H;
+  const bool flash = attention_supported(D);  // other head sizes keep the score matrix of every layer
   auto act = [&](__nv_bfloat16** p, size_t elems) { return aalloc((void**)p, elems * 2); };
   auto actf = [&](float** p, size_t elems) { return aalloc((void**)p, elems * 4); };
   if ((rc = act(&x0, T * C))) return rc;
   for (Layer& y : layers) {
-    if ((rc = act(&y.ln1o, T * C)) || (rc = act(&y.qkv_o, T * 3 * C)) || (rc = act(&y.Pm, BH * S * S)) ||
+    if ((rc = act(&y.ln1o, T * C)) || (rc = act(&y.qkv_o, T * 3 * C)) ||
+        (rc = flash ? actf(&y.rows, attention_rows_floats(B, S, H)) : act(&y.Pm, BH * S * S)) ||
         (rc = act(&y.att, T * C)) || (rc = act(&y.x2, T * C)) || (rc = act(&y.ln2o, T * C)) ||
         (rc = act(&y.h, T * 4 * C)) || (rc = act(&y.g, T * 4 * C)) || (rc = act(&y.xout, T * C)))
       return rc;
@@ -316,9 +321,10 @@ int Gpt2::alloc_activations(int B) {
   }
   if ((rc = act(&lnfo, T * C)) || (rc = act(&logits, T * Vpad))) return rc;
   if ((rc = actf(&lnf_mean, T)) || (rc = actf(&lnf_rstd, T)) || (rc = actf(&row_loss, T))) return rc;
-  if ((rc = act(&dxa, T * C)) || (rc = act(&dxb, T * C)) || (rc = act(&dqkv, T * 3 * C)) || (rc = act(&dP, BH * S * S)) ||
-      (rc = act(&Tbig, BH * S * S)) || (rc = act(&t1, T * C)) || (rc = act(&t2, T * C)) || (rc = act(&dh, T * 4 * C)) ||
+  if ((rc = act(&dxa, T * C)) || (rc = act(&dxb, T * C)) || (rc = act(&dqkv, T * 3 * C)) || (rc = act(&dh, T * 4 * C)) ||
       (rc = act(&dg, T * 4 * C)) || (rc = act(&datt, T * C)) || (rc = act(&dln, T * C)))
+    return rc;
+  if (!flash && ((rc = act(&dP, BH * S * S)) || (rc = act(&Tbig, BH * S * S)) || (rc = act(&t1, T * C)) || (rc = act(&t2, T * C))))
     return rc;
   act_batch = B;
   return SRT_OK;
@@ -334,6 +340,55 @@ int Gpt2::refresh() {
   return filter_transpose(SRT_BF16, pw(wte), WT + wte_wt_off, Vpad, 1, C, stream);
 }
 
+// Causal attention of one layer: qkv_o -> att. 64-channel heads take the fused kernel; other sizes go through the
+// score matrix.
+int Gpt2::attention_forward(Layer& y, int B, float scale) {
+  int rc;
+  if (attention_supported(D))
+    return attention_fwd({B, S, H, H, D}, y.qkv_o, y.qkv_o + C, y.qkv_o + 2 * C, 3LL * C, y.att, C, y.rows, scale, 1, stream);
+  // scores = Q K^T / sqrt(D), lower triangle only
+  BgemmDesc q = {S, S, D, H, B, 3LL * C, D, (long long)S * 3 * C, 3LL * C, D, (long long)S * 3 * C,
+                 S, (long long)S * S, (long long)H * S * S, scale, 1, 0};
+  if ((rc = bgemm_bf16(q, y.qkv_o, y.qkv_o + C, y.Pm, stream))) return rc;
+  if ((rc = causal_softmax_fwd(y.Pm, (int64_t)B * H, S, stream))) return rc;
+  // out = P V: B operand is V^T per head, [B][H][D][S]
+  if ((rc = batched_transpose(y.qkv_o + 2 * C, t1, S, D, 3LL * C, D, (long long)S * 3 * C, H, B, stream))) return rc;
+  BgemmDesc o = {S, D, S, H, B, S, (long long)S * S, (long long)H * S * S, S, (long long)D * S, (long long)H * D * S,
+                 C, D, (long long)S * C, 1.f, 0, 1};
+  return bgemm_bf16(o, y.Pm, t1, y.att, stream);
+}
+
+// datt -> dqkv.
+int Gpt2::attention_backward(Layer& y, int B, float scale) {
+  int rc;
+  if (attention_supported(D))
+    return attention_bwd_causal({B, S, H, H, D}, y.qkv_o, y.qkv_o + C, y.qkv_o + 2 * C, 3LL * C, datt, C, y.rows,
+                                dqkv, 3LL * C, dqkv + C, dqkv + 2 * C, 3LL * C, D, (long long)S * 3 * C, scale, stream);
+  // dP = dO V^T (lower triangle)
+  BgemmDesc dp = {S, S, D, H, B, C, D, (long long)S * C, 3LL * C, D, (long long)S * 3 * C,
+                  S, (long long)S * S, (long long)H * S * S, 1.f, 1, 0};
+  if ((rc = bgemm_bf16(dp, datt, y.qkv_o + 2 * C, dP, stream))) return rc;
+  // dV = P^T dO
+  if ((rc = batched_transpose(y.Pm, Tbig, S, S, S, (long long)S * S, (long long)H * S * S, H, B, stream, 1))) return rc;
+  if ((rc = batched_transpose(datt, t1, S, D, C, D, (long long)S * C, H, B, stream))) return rc;
+  BgemmDesc dv = {S, D, S, H, B, S, (long long)S * S, (long long)H * S * S, S, (long long)D * S, (long long)H * D * S,
+                  3LL * C, D, (long long)S * 3 * C, 1.f, 0, 2};
+  if ((rc = bgemm_bf16(dv, Tbig, t1, dqkv + 2 * C, stream))) return rc;
+  // dS = softmax backward, in place over dP
+  if ((rc = causal_softmax_bwd(y.Pm, dP, (int64_t)B * H, S, stream))) return rc;
+  // dQ = dS K / sqrt(D)
+  if ((rc = batched_transpose(y.qkv_o + C, t1, S, D, 3LL * C, D, (long long)S * 3 * C, H, B, stream))) return rc;
+  BgemmDesc dq = {S, D, S, H, B, S, (long long)S * S, (long long)H * S * S, S, (long long)D * S, (long long)H * D * S,
+                  3LL * C, D, (long long)S * 3 * C, scale, 0, 1};
+  if ((rc = bgemm_bf16(dq, dP, t1, dqkv, stream))) return rc;
+  // dK = dS^T Q / sqrt(D)
+  if ((rc = batched_transpose(dP, Tbig, S, S, S, (long long)S * S, (long long)H * S * S, H, B, stream, 1))) return rc;
+  if ((rc = batched_transpose(y.qkv_o, t2, S, D, 3LL * C, D, (long long)S * 3 * C, H, B, stream))) return rc;
+  BgemmDesc dk = dq;
+  dk.k_causal = 2;
+  return bgemm_bf16(dk, Tbig, t2, dqkv + C, stream);
+}
+
 int Gpt2::forward(int B) {
   const int64_t T = (int64_t)B * S;
   const float scale = 1.f / sqrtf((float)D);
@@ -345,16 +400,7 @@ int Gpt2::forward(int B) {
     if ((rc = checkpoint())) return rc;
     if ((rc = layernorm_fwd(x, pf(y.ln1_g), pf(y.ln1_b), y.ln1o, y.ln1_mean, y.ln1_rstd, T, C, cfg.ln_eps, stream))) return rc;
     if ((rc = linear_fwd(y.qkv, y.ln1o, y.qkv_o, nullptr, T))) return rc;
-    // scores = Q K^T / sqrt(D), lower triangle only
-    BgemmDesc q = {S, S, D, H, B, 3LL * C, D, (long long)S * 3 * C, 3LL * C, D, (long long)S * 3 * C,
-                   S, (long long)S * S, (long long)H * S * S, scale, 1, 0};
-    if ((rc = bgemm_bf16(q, y.qkv_o, y.qkv_o + C, y.Pm, stream))) return rc;
-    if ((rc = causal_softmax_fwd(y.Pm, (int64_t)B * H, S, stream))) return rc;
-    // out = P V: B operand is V^T per head, [B][H][D][S]
-    if ((rc = batched_transpose(y.qkv_o + 2 * C, t1, S, D, 3LL * C, D, (long long)S * 3 * C, H, B, stream))) return rc;
-    BgemmDesc o = {S, D, S, H, B, S, (long long)S * S, (long long)H * S * S, S, (long long)D * S, (long long)H * D * S,
-                   C, D, (long long)S * C, 1.f, 0, 1};
-    if ((rc = bgemm_bf16(o, y.Pm, t1, y.att, stream))) return rc;
+    if ((rc = attention_forward(y, B, scale))) return rc;
     if ((rc = linear_fwd(y.proj, y.att, y.x2, x, T))) return rc;                       // + residual
     if ((rc = layernorm_fwd(y.x2, pf(y.ln2_g), pf(y.ln2_b), y.ln2o, y.ln2_mean, y.ln2_rstd, T, C, cfg.ln_eps, stream))) return rc;
     if ((rc = linear_fwd(y.fc, y.ln2o, y.h, nullptr, T))) return rc;
@@ -408,29 +454,7 @@ int Gpt2::backward(int B, int global_batch) {
       return rc;  // dx_other = gradient w.r.t. x2
     // attention output projection
     if ((rc = linear_bwd(y.proj, dx_other, y.att, datt, T))) return rc;
-    // dP = dO V^T (lower triangle)
-    BgemmDesc dp = {S, S, D, H, B, C, D, (long long)S * C, 3LL * C, D, (long long)S * 3 * C,
-                    S, (long long)S * S, (long long)H * S * S, 1.f, 1, 0};
-    if ((rc = bgemm_bf16(dp, datt, y.qkv_o + 2 * C, dP, stream))) return rc;
-    // dV = P^T dO
-    if ((rc = batched_transpose(y.Pm, Tbig, S, S, S, (long long)S * S, (long long)H * S * S, H, B, stream, 1))) return rc;
-    if ((rc = batched_transpose(datt, t1, S, D, C, D, (long long)S * C, H, B, stream))) return rc;
-    BgemmDesc dv = {S, D, S, H, B, S, (long long)S * S, (long long)H * S * S, S, (long long)D * S, (long long)H * D * S,
-                    3LL * C, D, (long long)S * 3 * C, 1.f, 0, 2};
-    if ((rc = bgemm_bf16(dv, Tbig, t1, dqkv + 2 * C, stream))) return rc;
-    // dS = softmax backward, in place over dP
-    if ((rc = causal_softmax_bwd(y.Pm, dP, (int64_t)B * H, S, stream))) return rc;
-    // dQ = dS K / sqrt(D)
-    if ((rc = batched_transpose(y.qkv_o + C, t1, S, D, 3LL * C, D, (long long)S * 3 * C, H, B, stream))) return rc;
-    BgemmDesc dq = {S, D, S, H, B, S, (long long)S * S, (long long)H * S * S, S, (long long)D * S, (long long)H * D * S,
-                    3LL * C, D, (long long)S * 3 * C, scale, 0, 1};
-    if ((rc = bgemm_bf16(dq, dP, t1, dqkv, stream))) return rc;
-    // dK = dS^T Q / sqrt(D)
-    if ((rc = batched_transpose(dP, Tbig, S, S, S, (long long)S * S, (long long)H * S * S, H, B, stream, 1))) return rc;
-    if ((rc = batched_transpose(y.qkv_o, t2, S, D, 3LL * C, D, (long long)S * 3 * C, H, B, stream))) return rc;
-    BgemmDesc dk = dq;
-    dk.k_causal = 2;
-    if ((rc = bgemm_bf16(dk, Tbig, t2, dqkv + C, stream))) return rc;
+    if ((rc = attention_backward(y, B, scale))) return rc;
     // fused projection and the first LayerNorm; dx becomes the gradient w.r.t. the layer's input
     if ((rc = linear_bwd(y.qkv, dqkv, y.ln1o, dln, T))) return rc;
     if ((rc = join_side())) return rc;  // the next kernel overwrites dx, which this layer's first weight gradient read

@@ -4,7 +4,7 @@
 // projection tied to the token table, next-token cross-entropy, AdamW.
 //
 // Same layout as the GPT-2 executor: [tokens][features] bf16 rows, linear layers on the tcgen05 implicit-GEMM
-// kernels, attention products as batched tcgen05 GEMMs over 4-D tensor maps. Q, K and V live in one fused
+// kernels, attention over 4-D tensor maps (one kernel for 64-channel heads, batched GEMMs for other sizes). Q, K and V live in one fused
 // [tokens][(Hq + 2 Hkv) D] projection (their weights are adjacent rows of one matrix), gate and up in one
 // [tokens][2 F] projection. Several query heads read one KV head through the batch divisor of the GEMM; the
 // KV gradients are produced per query head and summed per group.
@@ -45,6 +45,7 @@ struct Qwen2 {
   struct Layer {
     int n1, n2;
     Lin qkv, o, gu, down;
+    float* rows;  // maximum, inverse sum and backward term of the score rows (64-channel heads, which keep no score matrix)
     __nv_bfloat16 *n1o, *qkv_o, *Pm, *att, *x2, *n2o, *gu_o, *act, *xout;
     float *z1, *r1, *z2, *r2;  // "mean" (zeros) and rstd of the two norms
   };
@@ -192,6 +193,8 @@ struct Qwen2 {
 
   int build();
   int transposes();
+  int attention_forward(Layer& y, int B, float scale);
+  int attention_backward(Layer& y, int B, float scale);
   int forward(int B);
   int backward(int B, int global_batch);
   srt_conv_desc lin_desc(int64_t T, int in, int out) const { return {(int)T, 1, 1, in, out, 1, 1, 1, 0, 1, 1}; }
@@ -301,6 +304,7 @@ int Qwen2::alloc_activations(int B) {
   int rc = free_activation_blocks();
   if (rc) return rc;
   const size_t T = (size_t)B * S, BH = (size_t)B * Hq;
+  const bool flash = attention_supported(D);  // other head sizes keep the score matrix of every layer
   auto act = [&](__nv_bfloat16** p, size_t elems) { return aalloc((void**)p, elems * 2); };
   auto actf = [&](float** p, size_t elems) { return aalloc((void**)p, elems * 4); };
   auto zeros = [&](float** p, size_t elems) -> int {  // the "mean" of an RMSNorm: zeros
@@ -311,18 +315,19 @@ int Qwen2::alloc_activations(int B) {
   };
   if ((rc = act(&x0, T * C))) return rc;
   for (Layer& y : layers) {
-    if ((rc = act(&y.n1o, T * C)) || (rc = act(&y.qkv_o, T * QKV)) || (rc = act(&y.Pm, BH * S * S)) ||
-        (rc = act(&y.att, T * Hq * D)) || (rc = act(&y.x2, T * C)) || (rc = act(&y.n2o, T * C)) ||
+    if ((rc = act(&y.n1o, T * C)) || (rc = act(&y.qkv_o, T * QKV)) ||
+        (rc = flash ? actf(&y.rows, attention_rows_floats(B, S, Hq)) : act(&y.Pm, BH * S * S)) || (rc = act(&y.att, T * Hq * D)) || (rc = act(&y.x2, T * C)) || (rc = act(&y.n2o, T * C)) ||
         (rc = act(&y.gu_o, T * 2 * F)) || (rc = act(&y.act, T * F)) || (rc = act(&y.xout, T * C)))
       return rc;
     if ((rc = zeros(&y.z1, T)) || (rc = actf(&y.r1, T)) || (rc = zeros(&y.z2, T)) || (rc = actf(&y.r2, T))) return rc;
   }
   if ((rc = act(&nfo, T * C)) || (rc = act(&logits, T * Vpad))) return rc;
   if ((rc = zeros(&zf, T)) || (rc = actf(&rf, T)) || (rc = actf(&row_loss, T))) return rc;
-  if ((rc = act(&dxa, T * C)) || (rc = act(&dxb, T * C)) || (rc = act(&dqkv, T * QKV)) || (rc = act(&dP, BH * S * S)) ||
-      (rc = act(&Tbig, BH * S * S)) || (rc = act(&t1, T * Hq * D)) || (rc = act(&t2, T * Hq * D)) ||
+  if ((rc = act(&dxa, T * C)) || (rc = act(&dxb, T * C)) || (rc = act(&dqkv, T * QKV)) || (rc = act(&t1, T * Hq * D)) ||
       (rc = act(&dkv_h, T * Hq * D)) || (rc = act(&dgu, T * 2 * F)) || (rc = act(&dact, T * F)) ||
       (rc = act(&datt, T * Hq * D)) || (rc = act(&dln, T * C)))
+    return rc;
+  if (!flash && ((rc = act(&dP, BH * S * S)) || (rc = act(&Tbig, BH * S * S)) || (rc = act(&t2, T * Hq * D))))
     return rc;
   act_batch = B;
   return SRT_OK;
@@ -336,11 +341,62 @@ int Qwen2::transposes() {
   return filter_transpose(SRT_BF16, Pw + params[emb].off, WT + emb_wt_off, Vpad, 1, C, stream);
 }
 
+// Causal grouped-query attention of one layer: qkv_o (rotated) -> att. 64-channel heads take the fused kernel; other
+// sizes go through the score matrix.
+int Qwen2::attention_forward(Layer& y, int B, float scale) {
+  const int KO = Hq * D, VO = (Hq + Hkv) * D;  // column offsets of K and V inside the fused projection
+  const long long SS = (long long)S * S;
+  int rc;
+  if (attention_supported(D))
+    return attention_fwd({B, S, Hq, Hkv, D}, y.qkv_o, y.qkv_o + KO, y.qkv_o + VO, QKV, y.att, KO, y.rows, scale, 1, stream);
+  BgemmDesc q = {S, S, D, Hq, B, QKV, D, (long long)S * QKV, QKV, D, (long long)S * QKV, S, SS, Hq * SS, scale, 1, 0, group};
+  if ((rc = bgemm_bf16(q, y.qkv_o, y.qkv_o + KO, y.Pm, stream))) return rc;
+  if ((rc = causal_softmax_fwd(y.Pm, (int64_t)B * Hq, S, stream))) return rc;
+  if ((rc = batched_transpose(y.qkv_o + VO, t1, S, D, QKV, D, (long long)S * QKV, Hkv, B, stream))) return rc;  // [B][Hkv][D][S]
+  BgemmDesc o = {S, D, S, Hq, B, S, SS, Hq * SS, S, (long long)D * S, (long long)Hkv * D * S, KO, D, (long long)S * KO,
+                 1.f, 0, 1, group};
+  return bgemm_bf16(o, y.Pm, t1, y.att, stream);
+}
+
+// datt -> dqkv (still rotated). dK and dV are made per query head and then summed over the heads of a group.
+int Qwen2::attention_backward(Layer& y, int B, float scale) {
+  const int KO = Hq * D, VO = (Hq + Hkv) * D;
+  const long long SS = (long long)S * S;
+  int rc;
+  if (attention_supported(D)) {
+    if ((rc = attention_bwd_causal({B, S, Hq, Hkv, D}, y.qkv_o, y.qkv_o + KO, y.qkv_o + VO, QKV, datt, KO, y.rows, dqkv, QKV, dkv_h, t1, D, (long long)S * D, (long long)Hq * S * D, scale, stream)))
+      return rc;
+    if ((rc = head_group_sum(t1, dqkv + VO, B, S, Hq, group, D, QKV, stream))) return rc;
+    return head_group_sum(dkv_h, dqkv + KO, B, S, Hq, group, D, QKV, stream);
+  }
+  BgemmDesc dp = {S, S, D, Hq, B, KO, D, (long long)S * KO, QKV, D, (long long)S * QKV, S, SS, Hq * SS, 1.f, 1, 0, group};
+  if ((rc = bgemm_bf16(dp, datt, y.qkv_o + VO, dP, stream))) return rc;
+  // dV per query head = P^T dO, then summed over the heads of a group
+  if ((rc = batched_transpose(y.Pm, Tbig, S, S, S, SS, Hq * SS, Hq, B, stream, 1))) return rc;
+  if ((rc = batched_transpose(datt, t1, S, D, KO, D, (long long)S * KO, Hq, B, stream))) return rc;       // dO^T [B][Hq][D][S]
+  BgemmDesc dv = {S, D, S, Hq, B, S, SS, Hq * SS, S, (long long)D * S, (long long)Hq * D * S, D, (long long)S * D,
+                  (long long)Hq * S * D, 1.f, 0, 2, 1};
+  if ((rc = bgemm_bf16(dv, Tbig, t1, dkv_h, stream))) return rc;                                           // [B][Hq][S][D]
+  if ((rc = head_group_sum(dkv_h, dqkv + VO, B, S, Hq, group, D, QKV, stream))) return rc;
+  if ((rc = causal_softmax_bwd(y.Pm, dP, (int64_t)B * Hq, S, stream))) return rc;
+  // dQ = dS K * scale (K of the group's KV head)
+  if ((rc = batched_transpose(y.qkv_o + KO, t1, S, D, QKV, D, (long long)S * QKV, Hkv, B, stream))) return rc;  // K^T [B][Hkv][D][S]
+  BgemmDesc dq = {S, D, S, Hq, B, S, SS, Hq * SS, S, (long long)D * S, (long long)Hkv * D * S, QKV, D, (long long)S * QKV,
+                  scale, 0, 1, group};
+  if ((rc = bgemm_bf16(dq, dP, t1, dqkv, stream))) return rc;
+  // dK per query head = dS^T Q * scale, summed per group
+  if ((rc = batched_transpose(dP, Tbig, S, S, S, SS, Hq * SS, Hq, B, stream, 1))) return rc;
+  if ((rc = batched_transpose(y.qkv_o, t2, S, D, QKV, D, (long long)S * QKV, Hq, B, stream))) return rc;        // Q^T [B][Hq][D][S]
+  BgemmDesc dk = {S, D, S, Hq, B, S, SS, Hq * SS, S, (long long)D * S, (long long)Hq * D * S, D, (long long)S * D,
+                  (long long)Hq * S * D, scale, 0, 2, 1};
+  if ((rc = bgemm_bf16(dk, Tbig, t2, dkv_h, stream))) return rc;
+  return head_group_sum(dkv_h, dqkv + KO, B, S, Hq, group, D, QKV, stream);
+}
+
 int Qwen2::forward(int B) {
   const int64_t T = (int64_t)B * S;
   const float scale = 1.f / sqrtf((float)D);
-  const int KO = Hq * D, VO = (Hq + Hkv) * D;  // column offsets of K and V inside the fused projection
-  const long long SS = (long long)S * S;
+  const int KO = Hq * D;  // column offset of K inside the fused projection
   int rc;
   if ((rc = join_side())) return rc;
   if ((rc = embedding_fwd(ids, pf(emb), nullptr, x0, T, S, C, stream))) return rc;
@@ -351,13 +407,7 @@ int Qwen2::forward(int B) {
     if ((rc = linear_fwd(y.qkv, y.n1o, y.qkv_o, nullptr, T))) return rc;
     if ((rc = rope_apply(y.qkv_o, T, S, Hq, D, QKV, cfg.rope_theta, 0, stream))) return rc;
     if ((rc = rope_apply(y.qkv_o + KO, T, S, Hkv, D, QKV, cfg.rope_theta, 0, stream))) return rc;
-    BgemmDesc q = {S, S, D, Hq, B, QKV, D, (long long)S * QKV, QKV, D, (long long)S * QKV, S, SS, Hq * SS, scale, 1, 0, group};
-    if ((rc = bgemm_bf16(q, y.qkv_o, y.qkv_o + KO, y.Pm, stream))) return rc;
-    if ((rc = causal_softmax_fwd(y.Pm, (int64_t)B * Hq, S, stream))) return rc;
-    if ((rc = batched_transpose(y.qkv_o + VO, t1, S, D, QKV, D, (long long)S * QKV, Hkv, B, stream))) return rc;  // [B][Hkv][D][S]
-    BgemmDesc o = {S, D, S, Hq, B, S, SS, Hq * SS, S, (long long)D * S, (long long)Hkv * D * S, KO, D, (long long)S * KO,
-                   1.f, 0, 1, group};
-    if ((rc = bgemm_bf16(o, y.Pm, t1, y.att, stream))) return rc;
+    if ((rc = attention_forward(y, B, scale))) return rc;
     if ((rc = linear_fwd(y.o, y.att, y.x2, x, T))) return rc;
     if ((rc = rmsnorm_fwd(y.x2, pf(y.n2), y.n2o, y.z2, y.r2, T, C, cfg.rms_eps, stream))) return rc;
     if ((rc = linear_fwd(y.gu, y.n2o, y.gu_o, nullptr, T))) return rc;
@@ -372,8 +422,7 @@ int Qwen2::forward(int B) {
 int Qwen2::backward(int B, int global_batch) {
   const int64_t T = (int64_t)B * S;
   const float scale = 1.f / sqrtf((float)D);
-  const int KO = Hq * D, VO = (Hq + Hkv) * D;
-  const long long SS = (long long)S * S;
+  const int KO = Hq * D;
   int rc;
   buckets.begin_backward();
   const float gscale = 1.f / ((float)global_batch * (float)(S - 1));
@@ -406,28 +455,7 @@ int Qwen2::backward(int B, int global_batch) {
       return rc;
     // attention
     if ((rc = linear_bwd(y.o, dx_other, y.att, datt, T))) return rc;
-    BgemmDesc dp = {S, S, D, Hq, B, KO, D, (long long)S * KO, QKV, D, (long long)S * QKV, S, SS, Hq * SS, 1.f, 1, 0, group};
-    if ((rc = bgemm_bf16(dp, datt, y.qkv_o + VO, dP, stream))) return rc;
-    // dV per query head = P^T dO, then summed over the heads of a group
-    if ((rc = batched_transpose(y.Pm, Tbig, S, S, S, SS, Hq * SS, Hq, B, stream, 1))) return rc;
-    if ((rc = batched_transpose(datt, t1, S, D, KO, D, (long long)S * KO, Hq, B, stream))) return rc;       // dO^T [B][Hq][D][S]
-    BgemmDesc dv = {S, D, S, Hq, B, S, SS, Hq * SS, S, (long long)D * S, (long long)Hq * D * S, D, (long long)S * D,
-                    (long long)Hq * S * D, 1.f, 0, 2, 1};
-    if ((rc = bgemm_bf16(dv, Tbig, t1, dkv_h, stream))) return rc;                                           // [B][Hq][S][D]
-    if ((rc = head_group_sum(dkv_h, dqkv + VO, B, S, Hq, group, D, QKV, stream))) return rc;
-    if ((rc = causal_softmax_bwd(y.Pm, dP, (int64_t)B * Hq, S, stream))) return rc;
-    // dQ = dS K * scale (K of the group's KV head)
-    if ((rc = batched_transpose(y.qkv_o + KO, t1, S, D, QKV, D, (long long)S * QKV, Hkv, B, stream))) return rc;  // K^T [B][Hkv][D][S]
-    BgemmDesc dq = {S, D, S, Hq, B, S, SS, Hq * SS, S, (long long)D * S, (long long)Hkv * D * S, QKV, D, (long long)S * QKV,
-                    scale, 0, 1, group};
-    if ((rc = bgemm_bf16(dq, dP, t1, dqkv, stream))) return rc;
-    // dK per query head = dS^T Q * scale, summed per group
-    if ((rc = batched_transpose(dP, Tbig, S, S, S, SS, Hq * SS, Hq, B, stream, 1))) return rc;
-    if ((rc = batched_transpose(y.qkv_o, t2, S, D, QKV, D, (long long)S * QKV, Hq, B, stream))) return rc;        // Q^T [B][Hq][D][S]
-    BgemmDesc dk = {S, D, S, Hq, B, S, SS, Hq * SS, S, (long long)D * S, (long long)Hq * D * S, D, (long long)S * D,
-                    (long long)Hq * S * D, scale, 0, 2, 1};
-    if ((rc = bgemm_bf16(dk, Tbig, t2, dkv_h, stream))) return rc;
-    if ((rc = head_group_sum(dkv_h, dqkv + KO, B, S, Hq, group, D, QKV, stream))) return rc;
+    if ((rc = attention_backward(y, B, scale))) return rc;
     // through the rotation (transposed), the fused projection and the first norm
     if ((rc = rope_apply(dqkv, T, S, Hq, D, QKV, cfg.rope_theta, 1, stream))) return rc;
     if ((rc = rope_apply(dqkv + KO, T, S, Hkv, D, QKV, cfg.rope_theta, 1, stream))) return rc;

@@ -17,6 +17,10 @@ class Gpt2ConfigC(C.Structure):
                 ("lr", _f), ("beta1", _f), ("beta2", _f), ("eps", _f), ("weight_decay", _f), ("ln_eps", _f)]
 
 
+class AttentionShapeC(C.Structure):
+    _fields_ = [(n, _i) for n in ("B", "S", "H", "Hkv", "D")]
+
+
 class BgemmDescC(C.Structure):
     _fields_ = [("M", _i), ("N", _i), ("K", _i), ("Z1", _i), ("Z2", _i)] + \
                [(n, C.c_longlong) for n in ("lda", "a_s1", "a_s2", "ldb", "b_s1", "b_s2", "ldd", "d_s1", "d_s2")] + \
@@ -48,6 +52,10 @@ register({
     "srt_gpt2_stream": (_vp, [_vp]),
     "srt_gpt2_memory_bytes": (_i64, [_vp]),
     "srt_gpt2_num_elements": (_i64, [_vp]),
+    "srt_attention_fwd": (None, [C.POINTER(AttentionShapeC), _vp, _vp, _vp, C.c_longlong, _vp, C.c_longlong, _vp, C.c_float,
+                                 _i, _vp]),
+    "srt_attention_bwd_causal": (None, [C.POINTER(AttentionShapeC), _vp, _vp, _vp, C.c_longlong, _vp, C.c_longlong, _vp, _vp,
+                                        C.c_longlong, _vp, _vp, C.c_longlong, C.c_longlong, C.c_longlong, C.c_float, _vp]),
     "srt_bgemm": (None, [C.POINTER(BgemmDescC), _vp, _vp, _vp, _vp]),
     "srt_layernorm_fwd": (None, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i, _f, _vp]),
     "srt_layernorm_bwd_scratch_bytes": (C.c_size_t, [_i]),
