@@ -39,3 +39,22 @@ def test_layernorm_variants(rows, cols, shift):
     assert rel(y, ref.detach()) < 4e-3
     assert rel(dx, xd.grad + add.double()) < 8e-3
     assert rel(dg, gd.grad) < 1e-5 and rel(db, bd.grad) < 1e-5
+
+
+@pytest.mark.parametrize("n", [1, 4, 7, 4099, 3_000_001])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_adamw_tails_and_alignment(n, shift):
+    g = torch.Generator(device="cuda").manual_seed(n)
+    new = lambda: torch.randn(n + shift, device="cuda", generator=g)[shift:]
+    p, gr, m, v = new(), new(), new(), new().abs()
+    pb = torch.empty(n + shift, device="cuda", dtype=torch.bfloat16)[shift:]
+    lr, b1, b2, eps, wd, step = 0.1, 0.9, 0.999, 1e-8, 0.01, 3
+    pd, gd, md, vd = (t.double() for t in (p, gr, m, v))
+    torch.cuda.synchronize()
+    call("srt_adamw", P(p), P(gr), P(m), P(v), P(pb), n, lr, b1, b2, eps, wd, step, None)
+    torch.cuda.synchronize()
+    md = b1 * md + (1 - b1) * gd
+    vd = b2 * vd + (1 - b2) * gd * gd
+    want = pd * (1 - lr * wd) - lr / (1 - b1 ** step) * md / (vd.sqrt() / (1 - b2 ** step) ** 0.5 + eps)
+    assert rel(m, md) < 1e-5 and rel(v, vd) < 1e-5 and rel(p, want) < 1e-4   # 1 - b2^3 in fp32 keeps five digits
+    assert torch.equal(pb, p.bfloat16())
