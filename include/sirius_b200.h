@@ -56,6 +56,11 @@ typedef struct srt_conv_epilogue {
 /* y[N,P,Q,K] = conv(x[N,H,W,C], w[K,R,S,C]). */
 int srt_conv_fprop(const srt_conv_desc* d, int dtype, int impl, const void* x, const void* w,
                    void* y, const srt_conv_epilogue* ep, void* stream);
+/* The same convolution with the epilogue of inference: y = act(conv(x, w) * scale + shift + addend), scale and shift per
+ * output channel (BatchNorm with running statistics, or a bias); any of the three may be null. act: 0 none, 1 ReLU,
+ * 2 GELU (erf form, bf16 only). The reduction may be split over a cluster of CTAs. */
+int srt_conv_fprop_infer(const srt_conv_desc* d, int dtype, int impl, const void* x, const void* w, void* y, const float* scale,
+                         const float* shift, const void* addend, int act, void* stream);
 /* dx[N,H,W,C] = conv^T(dy[N,P,Q,K], wt[C,R,S,K]); wt comes from srt_conv_filter_transpose. */
 int srt_conv_dgrad(const srt_conv_desc* d, int dtype, int impl, const void* dy, const void* wt,
                    void* dx, const srt_conv_epilogue* ep, void* stream);

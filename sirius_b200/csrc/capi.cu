@@ -117,6 +117,19 @@ int conv_fprop(const srt_conv_desc& d, int dtype, int impl, const void* x, const
   return conv_gather_gemm_simt(g, dtype, x, w, y, ep, st);
 }
 
+int conv_fprop_infer(const srt_conv_desc& d, int dtype, int impl, const void* x, const void* w, void* y, const InferEpilogue& ep,
+                     cudaStream_t st) {
+  int rc = check_desc(d);
+  if (rc) return rc;
+  SRT_REQUIRE(!(dtype == SRT_F32 && impl == SRT_IMPL_TCGEN05), "conv: tcgen05 path is bf16 only");
+  GatherGeom g = make_fprop_geom(d);
+  if (use_tc(dtype, impl)) return conv_infer_tc(g, x, w, y, ep, st);
+  SRT_REQUIRE(conv_fprop_infer_supported(d, dtype, impl) && conv_infer_simt_ok(g, x, w, y), "conv: no inference epilogue for this shape");
+  return conv_infer_simt(g, x, w, y, ep, st);
+}
+// bf16 on the CUDA cores is a cross-check without an epilogue of its own; fp32 has no GELU
+bool conv_fprop_infer_supported(const srt_conv_desc& d, int dtype, int impl) { return use_tc(dtype, impl) || dtype == SRT_F32; }
+
 bool conv_fprop_stats_supported(const srt_conv_desc& d, int dtype, int impl) {
   return use_tc(dtype, impl) && conv_col_stats_available() && d.C % 8 == 0 && d.K % 8 == 0;
 }
@@ -172,6 +185,13 @@ extern "C" {
 const char* srt_last_error(void) { return g_err; }
 const char* srt_version(void) { return "sirius_b200 0.1 (sm_100a)"; }
 
+int srt_conv_fprop_infer(const srt_conv_desc* d, int dtype, int impl, const void* x, const void* w, void* y, const float* scale,
+                         const float* shift, const void* addend, int act, void* stream) {
+  SRT_REQUIRE(d && x && w && y, "conv_fprop_infer: null argument");
+  CHECK_DTYPE(dtype);
+  SRT_REQUIRE(act >= ACT_NONE && act <= (dtype == SRT_BF16 ? ACT_GELU_ERF : ACT_RELU), "conv_fprop_infer: bad activation");
+  return conv_fprop_infer(*d, dtype, impl, x, w, y, {scale, shift, addend, act}, (cudaStream_t)stream);
+}
 int srt_conv_fprop(const srt_conv_desc* d, int dtype, int impl, const void* x, const void* w,
                    void* y, const srt_conv_epilogue* ep, void* stream) {
   SRT_REQUIRE(d && x && w && y, "conv_fprop: null argument");

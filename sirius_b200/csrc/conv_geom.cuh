@@ -76,7 +76,19 @@ inline GatherGeom make_dgrad_geom(const srt_conv_desc& d) {
   return g;
 }
 
+// Epilogue of a convolution in inference: y = act(conv * scale + shift + addend), scale and shift per output channel
+// (BatchNorm with running statistics, or a bias), any of the three may be null.
+enum { ACT_NONE = 0, ACT_RELU = 1, ACT_GELU_ERF = 2 };
+struct InferEpilogue {
+  const float *scale, *shift;
+  const void* addend;
+  int act;
+};
+
 // Declared here, defined in conv_simt.cu / igemm_tcgen05.cu.
+bool conv_infer_simt_ok(const GatherGeom& g, const void* src, const void* Bm, const void* D);
+int conv_infer_simt(const GatherGeom& g, const void* src, const void* Bm, void* D, const InferEpilogue& ep, cudaStream_t st);
+int conv_infer_tc(const GatherGeom& g, const void* src, const void* Bm, void* D, const InferEpilogue& ep, cudaStream_t st);
 int conv_gather_gemm_simt(const GatherGeom& g, int dtype, const void* src, const void* Bm, void* D,
                           const srt_conv_epilogue* ep, cudaStream_t st);
 int conv_wgrad_simt(const GatherGeom& g, int dtype, const void* dy, const void* x, float* dw,

@@ -2,7 +2,7 @@
 //
 // Two warp-specialised kernels:
 //
-//   igemm_fwd_persistent<BN, NS, PAIR>   fprop and dgrad.  D[m][n] = sum_k A(m,k) B[n][k]
+//   igemm_fwd_persistent<BN, NS, PAIR, INFER>   fprop and dgrad.  D[m][n] = sum_k A(m,k) B[n][k]
 //       Persistent: one CTA (or one CTA pair, cta_group::2) per SM walks output tiles of 128 (256 for a pair)
 //       rows x BN filters; 704 threads.
 //       A: 128 output positions x 64 reduction elements per stage, gathered from the NHWC source with 16-byte
@@ -542,6 +542,9 @@ struct PersistParams {
   // as double2 [m_tiles][Nout]. The BatchNorm that follows a convolution finalizes its statistics from these and
   // never reads the tensor for them.
   double* col_partial;
+  // Inference (template parameter INFER): y = act(acc * scale + bias + addend), see InferEpilogue
+  const float* scale;
+  int act;
 };
 
 enum WaitCode2 { W_MMA_TMEM_EMPTY = 5 };
@@ -581,7 +584,13 @@ __device__ __forceinline__ void cp_async_wait_lag(int lag) {
   }
 }
 
-template <int BN, int NS, bool PAIR>
+__device__ __forceinline__ float infer_act(float v, int act) {
+  if (act == ACT_RELU) return fmaxf(v, 0.f);
+  if (act == ACT_GELU_ERF) return 0.5f * v * (1.f + erff(v * 0.7071067811865476f));
+  return v;
+}
+
+template <int BN, int NS, bool PAIR, bool INFER>
 __global__ void __launch_bounds__(P_THREADS, 1)
 igemm_fwd_persistent(const PersistParams p, const __grid_constant__ CUtensorMap tmap_b,
                      const __grid_constant__ CUtensorMap tmap_a,
@@ -822,6 +831,10 @@ igemm_fwd_persistent(const PersistParams p, const __grid_constant__ CUtensorMap 
 #pragma unroll
             for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(acc[v * 8 + e]);
             if (col < g.Nout) {
+              if (INFER && p.scale) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] *= p.scale[col + e];
+              }
               if (p.bias) {
 #pragma unroll
                 for (int e = 0; e < 8; ++e) f[e] += p.bias[col + e];
@@ -840,6 +853,10 @@ igemm_fwd_persistent(const PersistParams p, const __grid_constant__ CUtensorMap 
 #pragma unroll
                 for (int e = 0; e < 8; ++e) f[e] += af[e];
               }
+              if (INFER) {
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] = infer_act(f[e], p.act);
+              }
             }
             Vec16<bf16> ov;
             ov.pack(f);
@@ -857,7 +874,7 @@ igemm_fwd_persistent(const PersistParams p, const __grid_constant__ CUtensorMap 
             bulk_commit_group();
           }
           if (issuer && grp == 0) SRT_STAMP(14);
-          if (p.col_partial != nullptr) {
+          if (!INFER && p.col_partial != nullptr) {
             // Column sums of the slab as it sits in the staging buffer. Warp w of the group takes columns
             // 16w..16w+15; a lane owns one column pair and a quarter of the rows, picked so that the 32 words
             // a warp reads at once fall into 32 different banks of the swizzled slab (the four row classes
@@ -1058,6 +1075,161 @@ igemm_fwd_persistent(const PersistParams p, const __grid_constant__ CUtensorMap 
     if (PAIR) tmem_dealloc_pair(tmem_base, 2 * BN);
     else tmem_dealloc(tmem_base, 2 * BN);
     if (lane == 0) SRT_STAMP(9);
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+// Inference at a small batch: few 128 x 64 output tiles and a reduction long enough to be shared. A cluster of S CTAs
+// works on one tile, each on its part of the k-blocks; the fp32 accumulators meet in shared memory (each CTA sends every
+// other its 64 / S columns), every CTA adds its columns in rank order, applies the epilogue and stores them. One tile on
+// one SM is bound by the serial chain of its k-blocks (a few hundred clocks each) and leaves most of the device idle: a
+// 196 x 256 layer with 36 k-blocks has 8 tiles. The convolutions of one ResNet-152 image: 1.71 ms of device time on the
+// persistent kernel (19.4 us for the long ones), 1.32 ms with the split, which is 8 us each, mostly launch, set-up and
+// the two cluster barriers; a sentence of 128 tokens through a 3072 x 768 layer: 26.3 us before, 11 us now.
+// No load is multicast; what crosses the cluster are the accumulators.
+constexpr int SPLIT_NS = 6;
+constexpr int SPLIT_STAGE_BYTES = A_STAGE_BYTES + 64 * BK * 2;
+constexpr size_t split_smem_bytes() { return 1024 + (size_t)SPLIT_NS * SPLIT_STAGE_BYTES + BM * 64 * 4 + (2 * SPLIT_NS + 1) * 8 + 16; }
+
+struct SplitParams {
+  GatherGeom g;
+  bf16* D;
+  const float *scale, *shift;
+  const bf16* addend;
+  int act, k_blocks, n_tiles, splits;
+  int a_tma, im_lower_w, im_lower_h, im_stride, im_cpt;  // as in PersistParams
+  int* status;
+};
+
+__global__ void __launch_bounds__(NTHREADS, 1)
+igemm_infer_split(const SplitParams p, const __grid_constant__ CUtensorMap tmap_b, const __grid_constant__ CUtensorMap tmap_a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* base = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  float* sums = (float*)(base + SPLIT_NS * SPLIT_STAGE_BYTES);  // [rank][16 / S column quads][128 rows][4]
+  uint64_t* full = (uint64_t*)((uint8_t*)sums + BM * 64 * 4);
+  uint64_t* empty = full + SPLIT_NS;
+  uint64_t* acc_full = empty + SPLIT_NS;
+  uint32_t* tmem_ptr = (uint32_t*)(acc_full + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const GatherGeom& g = p.g;
+  const int S = p.splits, rank = (int)cluster_ctarank(), tile = (int)blockIdx.x / S;
+  const int m0 = (tile / p.n_tiles) * BM, n0 = (tile % p.n_tiles) * 64;
+  const int kb0 = p.k_blocks * rank / S, nkb = p.k_blocks * (rank + 1) / S - kb0;  // at least one
+
+  if (tid == 0) {
+    for (int s = 0; s < SPLIT_NS; ++s) { mbar_init(smem_u32(&full[s]), 1); mbar_init(smem_u32(&empty[s]), 1); }
+    mbar_init(smem_u32(acc_full), 1);
+    mbar_fence_init();
+  }
+  if (warp == 4 && lane == 0) { tma_prefetch_desc(&tmap_b); tma_prefetch_desc(&tmap_a); }
+  if (warp == 5) { tmem_alloc(smem_u32(tmem_ptr), 64); tmem_relinquish(); }
+  tc_fence_before_sync();
+  __syncthreads();
+  cluster_sync_all();  // every CTA of the cluster runs before its shared memory is written
+  tc_fence_after_sync();
+  const uint32_t acc = *tmem_ptr;
+  pdl_enter();
+
+  if (warp < 4) {
+    mbar_wait(smem_u32(acc_full), 0u, p.status, W_EPI_TMEM);
+    tc_fence_after_sync();
+    const int row = warp * 32 + lane, quads = 16 / S;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t v[32];
+      tmem_ld_32x32b_x32(acc + ((uint32_t)(warp * 32) << 16) + (uint32_t)(h * 32), v);
+      tmem_ld_wait();
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int cq = h * 8 + q, to = cq / quads;
+        st_cluster_v4(map_to_cta(smem_u32(sums + ((rank * quads + cq - to * quads) * BM + row) * 4), (uint32_t)to), v[q * 4],
+                      v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
+      }
+    }
+  } else if (warp == 4) {
+    if (lane == 0) {
+      int iw0 = 0, ih0 = 0, in0 = 0, chunk = 0, tap_r = 0, tap_s = 0;
+      if (p.a_tma == 2) {
+        const RowCoord rc = decode_row(g, m0);
+        iw0 = rc.ow * p.im_stride + p.im_lower_w;
+        ih0 = rc.oh * p.im_stride + p.im_lower_h;
+        in0 = rc.n;
+        const int tap = kb0 / p.im_cpt;
+        chunk = kb0 - tap * p.im_cpt;
+        tap_r = tap / g.S;
+        tap_s = tap - tap_r * g.S;
+      }
+      for (int i = 0; i < nkb; ++i) {
+        const int s = i % SPLIT_NS;
+        if (!mbar_wait(smem_u32(&empty[s]), ((uint32_t)(i / SPLIT_NS) & 1u) ^ 1u, p.status, W_TMA_EMPTY)) break;
+        const uint32_t bar = smem_u32(&full[s]), dst = smem_u32(base + s * SPLIT_STAGE_BYTES);
+        mbar_arrive_expect_tx(bar, SPLIT_STAGE_BYTES);
+        tma_load_2d(dst + A_STAGE_BYTES, &tmap_b, bar, (kb0 + i) * BK, n0);
+        if (p.a_tma == 1) {
+          tma_load_2d(dst, &tmap_a, bar, (kb0 + i) * BK, m0);
+        } else {
+          tma_load_im2col_4d(dst, &tmap_a, bar, chunk * BK, iw0, ih0, in0, (uint16_t)tap_s, (uint16_t)tap_r);
+          if (++chunk == p.im_cpt) {
+            chunk = 0;
+            if (++tap_s == g.S) { tap_s = 0; ++tap_r; }
+          }
+        }
+      }
+    }
+  } else if (lane == 0) {
+    constexpr uint32_t idesc = make_idesc_bf16(BM, 64, 0, 0);
+    for (int i = 0; i < nkb; ++i) {
+      const int s = i % SPLIT_NS;
+      if (!mbar_wait(smem_u32(&full[s]), (uint32_t)(i / SPLIT_NS) & 1u, p.status, W_MMA_FULL)) break;
+      tc_fence_after_sync();
+      const uint32_t a0 = smem_u32(base + s * SPLIT_STAGE_BYTES), b0 = a0 + A_STAGE_BYTES;
+#pragma unroll
+      for (int k = 0; k < BK / 16; ++k)
+        umma_bf16(acc, make_smem_desc_sw128(a0 + k * 32, 0, 1024), make_smem_desc_sw128(b0 + k * 32, 0, 1024), idesc,
+                  (i | k) != 0 ? 1u : 0u);
+      umma_commit(smem_u32(&empty[s]));
+    }
+    umma_commit(smem_u32(acc_full));
+  }
+  __syncwarp();
+  cluster_sync_all();  // the partial sums of every rank are here (release on arrival, acquire on the wait)
+  if (tid < BM && m0 + tid < g.M) {
+    const int quads = 16 / S, m = m0 + tid;
+    for (int q = 0; q < quads; q += 2) {  // eight columns at a time (S is at most 8, so quads is even)
+      const int col = n0 + (rank * quads + q) * 4;
+      if (col >= g.Nout) break;  // Nout is a multiple of eight
+      float f[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = 0.f;
+      for (int r = 0; r < S; ++r)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const float4 v = *reinterpret_cast<const float4*>(sums + ((r * quads + q + e) * BM + tid) * 4);
+          f[e * 4] += v.x; f[e * 4 + 1] += v.y; f[e * 4 + 2] += v.z; f[e * 4 + 3] += v.w;
+        }
+      float af[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+      if (p.addend) {
+        Vec16<bf16> a;
+        a.load(p.addend + (size_t)m * g.Nout + col);
+        a.unpack(af);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        if (p.scale) f[e] *= p.scale[col + e];
+        if (p.shift) f[e] += p.shift[col + e];
+        f[e] = infer_act(f[e] + af[e], p.act);
+      }
+      Vec16<bf16> o;
+      o.pack(f);
+      o.store(p.D + (size_t)m * g.Nout + col);
+    }
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (warp == 5) {
+    __syncwarp();
+    tc_fence_after_sync();
+    tmem_dealloc(acc, 64);
   }
 }
 
@@ -1389,14 +1561,14 @@ int launch_wgrad_pair(const WgradParams& p, const CUtensorMap& tdy, const CUtens
   return SRT_OK;
 }
 
-template <int BN, int NS, bool PAIR>
+template <int BN, int NS, bool PAIR, bool INFER>
 int launch_persistent(const PersistParams& p, const CUtensorMap& tb, const CUtensorMap& ta,
                       const CUtensorMap& td, cudaStream_t st) {
   constexpr size_t smem = persist_smem_bytes<BN, NS, PAIR>();
   static_assert(smem <= 232448, "persistent igemm: shared memory budget exceeded");
   static bool configured = false;
   if (!configured) {
-    SRT_CHECK_CUDA(cudaFuncSetAttribute(igemm_fwd_persistent<BN, NS, PAIR>,
+    SRT_CHECK_CUDA(cudaFuncSetAttribute(igemm_fwd_persistent<BN, NS, PAIR, INFER>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = true;
   }
@@ -1424,7 +1596,7 @@ int launch_persistent(const PersistParams& p, const CUtensorMap& tb, const CUten
     const int tiles = p.m_tiles * p.n_tiles;
     cfg.gridDim = dim3(tiles < sm_count() ? tiles : sm_count());
   }
-  cudaLaunchKernelEx(&cfg, igemm_fwd_persistent<BN, NS, PAIR>, p, tb, ta, td);
+  cudaLaunchKernelEx(&cfg, igemm_fwd_persistent<BN, NS, PAIR, INFER>, p, tb, ta, td);
   SRT_LAUNCH_CHECK();
   return SRT_OK;
 }
@@ -1610,9 +1782,14 @@ void tc_set_conv_plan(int gather, int tile_n, int pair) {
   g_force_pair = pair;
 }
 
+// INFER: `ep` holds the bias and the addend, `infer` the rest of the inference epilogue.
+template <bool INFER>
 static int conv_gather_gemm_tc_persistent(const GatherGeom& g, const void* src, const void* Bm, void* D,
-                                          const srt_conv_epilogue* ep, cudaStream_t st, double* col_partial = nullptr) {
+                                          const srt_conv_epilogue* ep, cudaStream_t st, double* col_partial = nullptr,
+                                          const InferEpilogue* infer = nullptr) {
   PersistParams p;
+  p.scale = infer ? infer->scale : nullptr;
+  p.act = infer ? infer->act : ACT_NONE;
   p.g = g;
   p.col_partial = col_partial;
   p.src = (const bf16*)src;
@@ -1671,14 +1848,14 @@ static int conv_gather_gemm_tc_persistent(const GatherGeom& g, const void* src, 
     return l < 1 ? 1 : l;
   };
   if (pair) {
-    if (bn == 128) { p.gather_lag = lag(6); return launch_persistent<128, 6, true>(p, tb, ta, td, st); }
+    if (bn == 128) { p.gather_lag = lag(6); return launch_persistent<128, 6, true, INFER>(p, tb, ta, td, st); }
     p.gather_lag = lag(5);
-    return launch_persistent<256, 5, true>(p, tb, ta, td, st);
+    return launch_persistent<256, 5, true, INFER>(p, tb, ta, td, st);
   }
-  if (bn == 64) { p.gather_lag = lag(6); return launch_persistent<64, 6, false>(p, tb, ta, td, st); }
-  if (bn == 128) { p.gather_lag = lag(5); return launch_persistent<128, 5, false>(p, tb, ta, td, st); }
+  if (bn == 64) { p.gather_lag = lag(6); return launch_persistent<64, 6, false, INFER>(p, tb, ta, td, st); }
+  if (bn == 128) { p.gather_lag = lag(5); return launch_persistent<128, 5, false, INFER>(p, tb, ta, td, st); }
   p.gather_lag = lag(3);
-  return launch_persistent<256, 3, false>(p, tb, ta, td, st);
+  return launch_persistent<256, 3, false, INFER>(p, tb, ta, td, st);
 }
 
 int conv_gather_gemm_tc(const GatherGeom& g, const void* src, const void* Bm, void* D,
@@ -1686,7 +1863,72 @@ int conv_gather_gemm_tc(const GatherGeom& g, const void* src, const void* Bm, vo
   SRT_REQUIRE(g.src_c % 8 == 0 && g.Nout % 8 == 0,
               "tcgen05 conv: channel counts (%d, %d) must be multiples of 8", g.src_c, g.Nout);
   SRT_REQUIRE(((uintptr_t)src & 15) == 0 && ((uintptr_t)D & 15) == 0, "tcgen05 conv: unaligned tensor");
-  return conv_gather_gemm_tc_persistent(g, src, Bm, D, ep, st);
+  return conv_gather_gemm_tc_persistent<false>(g, src, Bm, D, ep, st);
+}
+
+// Cluster size of the split kernel, 1 where the persistent kernel is the better one: the tiles times the cluster must fit
+// the device in one wave (a second wave of clusters would double the time that the split is there to shorten), every CTA
+// gets at least two k-blocks (a k-block less per CTA saves less than the cluster barriers cost), and both operands come
+// by TMA. A partition of the device may have no room for a cluster: it takes the persistent kernel.
+static int infer_splits(const GatherGeom& g, int a_tma) {
+  if (!a_tma || sm_limit() != 0) return 1;
+  const int tiles = ceil_div(g.M, BM) * ceil_div(g.Nout, 64), nkb = ceil_div(g.Kg, BK);
+  int s = 8;
+  while (s > 1 && (tiles * s > sm_count() || nkb < 2 * s)) s /= 2;
+  return s;
+}
+
+int conv_infer_tc(const GatherGeom& g, const void* src, const void* Bm, void* D, const InferEpilogue& ep, cudaStream_t st) {
+  SRT_REQUIRE(!g.dgrad && g.src_c % 8 == 0 && g.Nout % 8 == 0,
+              "tcgen05 conv: channel counts (%d, %d) must be multiples of 8", g.src_c, g.Nout);
+  SRT_REQUIRE((((uintptr_t)src | (uintptr_t)D | (uintptr_t)ep.addend) & 15) == 0, "tcgen05 conv: unaligned tensor");
+  SplitParams p;
+  const bool plain = g.R == 1 && g.S == 1 && g.stride == 1 && g.pad == 0;
+  p.a_tma = g_force_gather ? 0 : plain ? 1 : (im2col_ok(g) && g_im2col_enabled) ? 2 : 0;
+  p.splits = infer_splits(g, p.a_tma);
+  if (p.splits == 1) {
+    const srt_conv_epilogue e = {ep.shift, ep.addend};
+    return conv_gather_gemm_tc_persistent<true>(g, src, Bm, D, &e, st, nullptr, &ep);
+  }
+  p.g = g;
+  p.D = (bf16*)D;
+  p.scale = ep.scale; p.shift = ep.shift; p.addend = (const bf16*)ep.addend; p.act = ep.act;
+  p.k_blocks = ceil_div(g.Kg, BK);
+  p.n_tiles = ceil_div(g.Nout, 64);
+  p.im_lower_w = p.im_lower_h = 0;
+  p.im_stride = p.im_cpt = 1;
+  if (p.a_tma == 2) {
+    const Im2colBox b = im2col_box(g);
+    p.im_lower_w = b.lower_w; p.im_lower_h = b.lower_h; p.im_stride = b.stride;
+    p.im_cpt = g.src_c / BK;
+  }
+  p.status = status_ptr();
+  SRT_REQUIRE(p.status != nullptr, "tcgen05 status word unavailable");
+  CUtensorMap tb, ta;
+  int rc = make_tmap_2d(&tb, Bm, (uint64_t)g.Nout, (uint64_t)g.Kg, 64);
+  if (rc != SRT_OK) return rc;
+  rc = p.a_tma == 1 ? make_tmap_2d(&ta, src, (uint64_t)g.M, (uint64_t)g.Kg, (uint32_t)BM) : make_tmap_im2col(&ta, src, g, (uint32_t)BM);
+  if (rc != SRT_OK) return rc;
+  constexpr size_t smem = split_smem_bytes();
+  static_assert(smem <= 232448, "split igemm: shared memory budget exceeded");
+  SRT_CHECK_CUDA(cudaFuncSetAttribute(igemm_infer_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ceil_div(g.M, BM) * p.n_tiles * p.splits);
+  cfg.blockDim = dim3(NTHREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = (pdl_big_kernels() && (pdl_classes() & PDL_GEMM) != 0) ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = p.splits;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  SRT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, igemm_infer_split, p, tb, ta));
+  SRT_LAUNCH_CHECK();
+  return SRT_OK;
 }
 
 // Convolution whose epilogue also leaves the per-tile column sums for the BatchNorm that follows
@@ -1702,7 +1944,7 @@ int conv_gather_gemm_tc_stats(const GatherGeom& g, const void* src, const void* 
               "tcgen05 conv: column-sum buffer missing, unaligned or too small (%zu < %zu)", col_partial_bytes,
               conv_col_stats_bytes(g.M, g.Nout));
   if (slabs) *slabs = ceil_div(g.M, BM);
-  return conv_gather_gemm_tc_persistent(g, src, Bm, D, ep, st, col_partial);
+  return conv_gather_gemm_tc_persistent<false>(g, src, Bm, D, ep, st, col_partial);
 }
 
 static size_t wgrad_plan_bytes(const GatherGeom& g, const WgradPlan& w) {

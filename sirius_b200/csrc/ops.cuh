@@ -13,8 +13,13 @@ int bn_finalize(const void* partial, int slabs, int C, int64_t rows, const float
 int bn_stats(int dtype, const void* z, int64_t rows, int C, const float* gamma, const float* beta,
              float eps, float momentum, float* rm, float* rv, float* mean, float* invstd,
              float* scale, float* shift, void* scratch, size_t scratch_bytes, cudaStream_t st);
-int bn_eval_params(const float* gamma, const float* beta, const float* rmean, const float* rvar, float eps, int C,
-                   float* scale, float* shift, cudaStream_t st);
+// scale and shift of inference-mode BatchNorm for a list of layers, 128 of them per launch.
+struct BnEvalLayer {
+  const float *gamma, *beta, *rmean, *rvar;
+  float *scale, *shift;
+  int C;
+};
+int bn_eval_params(const BnEvalLayer* layers, int n, float eps, cudaStream_t st);
 int bn_stats_static(int dtype, const void* z, int64_t rows, int C, const float* gamma,
                     const float* beta, float eps, float momentum, float* rm, float* rv, float* mean,
                     float* invstd, float* scale, float* shift, cudaStream_t st);
@@ -68,6 +73,10 @@ int parity_interleave(int dtype, const void* c00, const void* c01, const void* c
 // Convolution front ends: validate, pick the kernel family, launch.
 int conv_fprop(const srt_conv_desc& d, int dtype, int impl, const void* x, const void* w, void* y,
                const srt_conv_epilogue* ep, cudaStream_t st);
+// fprop with the epilogue of inference (see InferEpilogue); may split the reduction over a cluster of CTAs.
+bool conv_fprop_infer_supported(const srt_conv_desc& d, int dtype, int impl);
+int conv_fprop_infer(const srt_conv_desc& d, int dtype, int impl, const void* x, const void* w, void* y, const InferEpilogue& ep,
+                     cudaStream_t st);
 int conv_dgrad(const srt_conv_desc& d, int dtype, int impl, const void* dy, const void* wt,
                void* dx, const srt_conv_epilogue* ep, cudaStream_t st);
 // fprop that also leaves the column sums of y for bn_finalize (bf16 tensor-core path only; ask

@@ -49,7 +49,7 @@ struct Bert {
   std::vector<void*> act_blocks;
   size_t act_bytes = 0;
   __nv_bfloat16 *emb = nullptr, *xa = nullptr, *xb = nullptr, *qkv = nullptr, *Pm = nullptr, *vt = nullptr, *att = nullptr,
-                *t1 = nullptr, *sa = nullptr, *h1 = nullptr, *g1 = nullptr;
+                *t1 = nullptr, *sa = nullptr, *g1 = nullptr;
   float *mean = nullptr, *rstd = nullptr;
   const __nv_bfloat16* out = nullptr;  // last hidden state of the latest forward
 
@@ -102,9 +102,8 @@ struct Bert {
   float* pf(int i) { return P + params[i].off; }
   __nv_bfloat16* pw(int i) { return Pw + params[i].off; }
   srt_conv_desc lin_desc(int64_t T, int in, int o) const { return {(int)T, 1, 1, in, o, 1, 1, 1, 0, 1, 1}; }
-  int linear(int w, int b, int in, int o, const void* x, void* y, const void* residual, int64_t T) {
-    srt_conv_epilogue ep = {pf(b), residual};
-    return conv_fprop(lin_desc(T, in, o), SRT_BF16, SRT_IMPL_AUTO, x, pw(w), y, &ep, stream);
+  int linear(int w, int b, int in, int o, const void* x, void* y, const void* residual, int64_t T, int act = ACT_NONE) {
+    return conv_fprop_infer(lin_desc(T, in, o), SRT_BF16, SRT_IMPL_AUTO, x, pw(w), y, {nullptr, pf(b), residual, act}, stream);
   }
   int build();
   int alloc_activations();
@@ -161,7 +160,7 @@ int Bert::alloc_activations() {
   auto act = [&](__nv_bfloat16** p, size_t elems) { return aalloc((void**)p, elems * 2); };
   if ((rc = act(&emb, T * C)) || (rc = act(&xa, T * C)) || (rc = act(&xb, T * C)) || (rc = act(&qkv, T * 3 * C)) ||
       (rc = act(&att, T * C)) || (rc = act(&t1, T * C)) ||
-      (rc = act(&sa, T * C)) || (rc = act(&h1, T * F)) || (rc = act(&g1, T * F)))
+      (rc = act(&sa, T * C)) || (rc = act(&g1, T * F)))
     return rc;
   // head sizes other than 64 go through the score matrix
   if (!attention_supported(D) && ((rc = act(&Pm, BH * S * S)) || (rc = act(&vt, T * C)))) return rc;
@@ -195,8 +194,7 @@ int Bert::forward(int B) {
     }
     if ((rc = linear(y.wo, y.bo, C, C, att, t1, x, T))) return rc;                                   // + residual
     if ((rc = layernorm_fwd(t1, pf(y.ln1_g), pf(y.ln1_b), sa, mean, rstd, T, C, cfg.ln_eps, stream))) return rc;
-    if ((rc = linear(y.w1, y.b1, C, F, sa, h1, nullptr, T))) return rc;
-    if ((rc = gelu_erf_fwd(h1, g1, T * F, stream))) return rc;
+    if ((rc = linear(y.w1, y.b1, C, F, sa, g1, nullptr, T, ACT_GELU_ERF))) return rc;
     if ((rc = linear(y.w2, y.b2, F, C, g1, t1, sa, T))) return rc;                                   // + residual
     if ((rc = layernorm_fwd(t1, pf(y.ln2_g), pf(y.ln2_b), nxt, mean, rstd, T, C, cfg.ln_eps, stream))) return rc;
     std::swap(x, nxt);

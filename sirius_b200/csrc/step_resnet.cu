@@ -802,13 +802,15 @@ int Step::forward(int B) {
       return timed(SRT_PROF_NORM, abytes * (residual ? 3 : 2) + (bits ? abytes / 16 : 0), [&] {
         return bn_apply(dt, u.z, residual, u.y, rows, u.bn.C, u.bn.scale, u.bn.shift, u.relu, stream, bits); });
     }
+    if (eval_mode && conv_fprop_infer_supported(d, dt, impl)) {
+      // inference: BatchNorm with the running statistics, the residual and the ReLU ride in the convolution's epilogue
+      const InferEpilogue ep = {u.bn.scale, u.bn.shift, residual, u.relu ? ACT_RELU : ACT_NONE};
+      return timed(SRT_PROF_CONV, flops, [&] { return conv_fprop_infer(d, dt, impl, in, pw(u.conv.w), u.y, ep, stream); });
+    }
     if ((r = timed(SRT_PROF_CONV, flops, [&] { return conv_fprop(d, dt, impl, in, pw(u.conv.w), u.z, nullptr, stream); })))
       return r;
     if (eval_mode) {
-      // inference: normalise with the running statistics (scale/shift prepared by bn_eval_params)
-      if ((r = bn_eval_params(pf(u.bn.gamma), pf(u.bn.beta), bf_(u.bn.rmean), bf_(u.bn.rvar), cfg.bn_eps, u.bn.C,
-                              u.bn.scale, u.bn.shift, stream)))
-        return r;
+      // scale and shift were prepared below, for all layers at once
     } else if (fused_bn && bn_fused_pays(dt, rows, u.bn.C, 0)) {
       // statistics, finalize and apply in one cooperative launch
       return timed(SRT_PROF_NORM, abytes * (residual ? 3 : 2), [&] {
@@ -828,6 +830,20 @@ int Step::forward(int B) {
   if ((rc = timed(SRT_PROF_OTHER, img_px * (3 * 4 + kStemCpad * esz), [&] {
         return nchw_to_nhwc(dt, stage_images, x0, B, 3, cfg.image, cfg.image, kStemCpad, stream); })))
     return rc;
+  if (eval_mode) {
+    std::vector<BnEvalLayer> layers;
+    auto add = [&](Unit& u) {
+      layers.push_back({pf(u.bn.gamma), pf(u.bn.beta), bf_(u.bn.rmean), bf_(u.bn.rvar), u.bn.scale, u.bn.shift, u.bn.C});
+    };
+    add(stem);
+    for (auto& k : blocks) {
+      add(k.u1);
+      add(k.u2);
+      if (k.has_ds) add(k.ds);
+      add(k.u3);
+    }
+    if ((rc = bn_eval_params(layers.data(), (int)layers.size(), cfg.bn_eps, stream))) return rc;
+  }
   if ((rc = run_unit(stem, x0, nullptr))) return rc;
   const double pool_in = (double)B * stem.P * stem.Q * 64 * esz;
   if ((rc = timed(SRT_PROF_OTHER, pool_in * 1.25 + pool_in / 4 / esz, [&] {
@@ -851,6 +867,8 @@ int Step::forward(int B) {
   srt_conv_desc fd = {B, 1, 1, feat_C, cfg.num_classes, 1, 1, 1, 0, 1, 1};
   srt_conv_epilogue ep = {pf(fc_b), nullptr};
   return timed(SRT_PROF_CONV, 2.0 * B * feat_C * cfg.num_classes, [&] {
+    if (eval_mode && conv_fprop_infer_supported(fd, dt, impl))
+      return conv_fprop_infer(fd, dt, impl, avg, pw(fc_w), logits, {nullptr, pf(fc_b), nullptr, ACT_NONE}, stream);
     return conv_fprop(fd, dt, impl, avg, pw(fc_w), logits, &ep, stream); });
 }
 
