@@ -474,6 +474,13 @@ size_t srt_layernorm_bwd_scratch_bytes(int C);
 int srt_layernorm_bwd(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd,
                       const void* addend, void* dx, float* dgamma, float* dbeta, int64_t rows, int C, void* scratch,
                       size_t scratch_bytes, void* stream);
+/* Shifted-window attention of 32-channel heads in windows of at most 64 tokens: qkv [B*Hs*Ws][3][heads][32] in natural token
+ * order, table [(2 WS - 1)^2][heads] relative-position biases. Backward recomputes the probabilities and writes dqkv and
+ * dS [windows][heads][WS*WS][ld] (ld a multiple of 8, WS*WS..64), from which the table's gradient is summed. */
+int srt_window_attention_fwd(const void* qkv, const float* table, void* out, int B, int Hs, int Ws, int WS, int shift, int heads,
+                             int D, float scale, void* stream);
+int srt_window_attention_bwd(const void* qkv, const float* table, const void* dout, void* dqkv, void* dS, int ld, int B, int Hs,
+                             int Ws, int WS, int shift, int heads, int D, float scale, void* stream);
 int srt_gelu_fwd(const void* x, void* y, int64_t n, void* stream);
 int srt_gelu_bwd(const void* dy, const void* x, void* dx, int64_t n, void* stream);
 int srt_causal_softmax_fwd(void* scores, int64_t Z, int S, void* stream);

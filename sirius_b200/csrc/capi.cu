@@ -450,6 +450,16 @@ int srt_layernorm_bwd(const void* dy, const void* x, const float* gamma, const f
   return layernorm_bwd(dy, x, gamma, mean, rstd, addend, dx, dgamma, dbeta, rows, C, scratch, scratch_bytes,
                        (cudaStream_t)stream);
 }
+int srt_window_attention_fwd(const void* qkv, const float* table, void* out, int B, int Hs, int Ws, int WS, int shift, int heads,
+                             int D, float scale, void* stream) {
+  SRT_REQUIRE(qkv && table && out, "window_attention_fwd: null argument");
+  return window_attention_fwd(qkv, table, out, {B, Hs, Ws, WS, shift}, heads, D, scale, (cudaStream_t)stream);
+}
+int srt_window_attention_bwd(const void* qkv, const float* table, const void* dout, void* dqkv, void* dS, int ld, int B, int Hs,
+                             int Ws, int WS, int shift, int heads, int D, float scale, void* stream) {
+  SRT_REQUIRE(qkv && table && dout && dqkv && dS, "window_attention_bwd: null argument");
+  return window_attention_bwd(qkv, table, dout, dqkv, dS, ld, {B, Hs, Ws, WS, shift}, heads, D, scale, (cudaStream_t)stream);
+}
 int srt_gelu_fwd(const void* x, void* y, int64_t n, void* stream) {
   SRT_REQUIRE(x && y, "gelu_fwd: null argument");
   return gelu_fwd(x, y, n, (cudaStream_t)stream);

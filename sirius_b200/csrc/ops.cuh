@@ -159,6 +159,14 @@ int gelu_erf_fwd(const void* x, void* y, int64_t n, cudaStream_t st);
 int gelu_erf_bwd(const void* dy, const void* x, void* dx, int64_t n, cudaStream_t st);
 // Shifted-window attention (Swin): tokens in natural [B][Hs][Ws] order, windows of WS x WS, cyclic shift.
 struct WindowShape { int B, Hs, Ws, WS, shift; };
+// Fused attention of 32-channel heads in windows of at most 64 tokens, from and to the natural [tokens][3][heads][32]
+// projection (window_attention.cu); table: relative-position biases [(2 WS - 1)^2][heads]. Backward writes dqkv and, for
+// relbias_grad, dS [windows][heads][WS * WS][ld]. Other shapes go through the window_* functions below.
+inline bool window_attention_supported(int WS, int D) { return D == 32 && WS * WS <= 64; }
+int window_attention_fwd(const void* qkv, const float* table, void* out, const WindowShape& w, int heads, int D, float scale,
+                         cudaStream_t st);
+int window_attention_bwd(const void* qkv, const float* table, const void* dout, void* dqkv, void* dS, int ld, const WindowShape& w,
+                         int heads, int D, float scale, cudaStream_t st);
 int window_permute(const void* in, void* out, const WindowShape& w, int C, int to_natural, cudaStream_t st);
 int window_qkv(void* nat, void* qw, void* kw, void* vw, const WindowShape& w, int heads, int D, int to_natural,
                cudaStream_t st);

@@ -5,10 +5,10 @@
 //
 // Data layout: tokens stay in the natural [batch][row][col] order as [tokens][features] bf16 rows, so every
 // linear layer is a 1x1 convolution on the tcgen05 implicit-GEMM kernels (bias / residual in the epilogue).
-// Only attention works on windows: Q, K, V are regrouped to [window][head][49][D] (the cyclic shift is folded
-// into that permutation), the four small products per window and head are batched tcgen05 GEMMs over all
-// windows at once, and the result goes back through the inverse permutation. Rows of 49 are padded to 56
-// wherever they are a reduction or output axis.
+// Only attention works on windows: one kernel each way gathers the windows (the cyclic shift is folded into the
+// gather) and scatters the result. Head sizes other than 32 regroup Q, K, V to [window][head][49][D], run the
+// small products per window and head as batched tcgen05 GEMMs over all windows at once, and go back through the
+// inverse permutation. Rows of 49 are padded to 56 wherever they are a reduction or output axis.
 #include <string.h>
 
 #include <string>
@@ -43,7 +43,8 @@ struct Swin {
     int C, heads, D, Hs, shift;
     int n1g, n1b, n2g, n2b, table;
     Lin qkv, proj, fc, fc2;
-    __nv_bfloat16 *ln1o, *qw, *kw, *vw, *Pm, *att, *x2, *ln2o, *h, *g, *xout;
+    bool fused;          // attention straight on the projection (qkv_o); otherwise on windowed copies (qw, kw, vw, Pm)
+    __nv_bfloat16 *ln1o, *qkv_o, *qw, *kw, *vw, *Pm, *att, *x2, *ln2o, *h, *g, *xout;
     float *m1, *r1, *m2, *r2;
   };
   struct Merge {
@@ -225,11 +226,18 @@ int Swin::build() {
   const size_t T0 = B * S0 * S0;
   if ((rc = act(&x_img, B * I * I * 8)) || (rc = act(&e0, T0 * cfg.embed)) || (rc = act(&x0, T0 * cfg.embed))) return rc;
   if ((rc = dalloc(&pe_m, T0 * 4)) || (rc = dalloc(&pe_r, T0 * 4))) return rc;
+  bool all_fused = true;
   size_t maxTC = T0 * cfg.embed, maxZLL = 0, maxTable = 0;
   for (Blk& k : blocks) {
     const size_t T = B * k.Hs * k.Hs, TC = T * k.C, Z = T / L * k.heads;
-    if ((rc = act(&k.ln1o, TC)) || (rc = act(&k.qw, TC)) || (rc = act(&k.kw, TC)) || (rc = act(&k.vw, TC)) ||
-        (rc = act(&k.Pm, Z * L * LP)) || (rc = act(&k.att, TC)) || (rc = act(&k.x2, TC)) || (rc = act(&k.ln2o, TC)) ||
+    k.fused = window_attention_supported(WS, k.D);
+    if (k.fused) {
+      if ((rc = act(&k.qkv_o, 3 * TC))) return rc;
+    } else {
+      if ((rc = act(&k.qw, TC)) || (rc = act(&k.kw, TC)) || (rc = act(&k.vw, TC)) || (rc = act(&k.Pm, Z * L * LP))) return rc;
+      all_fused = false;
+    }
+    if ((rc = act(&k.ln1o, TC)) || (rc = act(&k.att, TC)) || (rc = act(&k.x2, TC)) || (rc = act(&k.ln2o, TC)) ||
         (rc = act(&k.h, 4 * TC)) || (rc = act(&k.g, 4 * TC)) || (rc = act(&k.xout, TC)))
       return rc;
     if ((rc = dalloc(&k.m1, T * 4)) || (rc = dalloc(&k.r1, T * 4)) || (rc = dalloc(&k.m2, T * 4)) || (rc = dalloc(&k.r2, T * 4)))
@@ -252,9 +260,10 @@ int Swin::build() {
     return rc;
   const size_t padTC = maxTC * LP / L + 4096;  // [Z][D][LP] buffers
   if ((rc = act(&dxa, maxTC)) || (rc = act(&dxb, maxTC)) || (rc = act(&dqkv, 3 * maxTC)) || (rc = act(&dP, maxZLL)) ||
-      (rc = act(&tP, maxZLL)) || (rc = act(&tA, padTC)) || (rc = act(&tB, padTC)) || (rc = act(&dOh, maxTC)) ||
-      (rc = act(&dqw, maxTC)) || (rc = act(&dkw, maxTC)) || (rc = act(&dvw, maxTC)) || (rc = act(&dh, 4 * maxTC)) ||
-      (rc = act(&dg, 4 * maxTC)) || (rc = act(&datt, maxTC)) || (rc = act(&dln, 4 * maxTC)) || (rc = act(&ow, maxTC)))
+      (rc = act(&dh, 4 * maxTC)) || (rc = act(&dg, 4 * maxTC)) || (rc = act(&datt, maxTC)) || (rc = act(&dln, 4 * maxTC)))
+    return rc;
+  if (!all_fused && ((rc = act(&tP, maxZLL)) || (rc = act(&tA, padTC)) || (rc = act(&tB, padTC)) || (rc = act(&dOh, maxTC)) ||
+                     (rc = act(&dqw, maxTC)) || (rc = act(&dkw, maxTC)) || (rc = act(&dvw, maxTC)) || (rc = act(&ow, maxTC))))
     return rc;
   size_t sb = layernorm_bwd_scratch_bytes(4 * Cf);
   if (colsum_scratch_bytes(4 * Cf) > sb) sb = colsum_scratch_bytes(4 * Cf);
@@ -307,18 +316,23 @@ int Swin::block_fwd(Blk& k, const __nv_bfloat16* x, int B) {
   const float scale = 1.f / sqrtf((float)D);
   int rc;
   if ((rc = layernorm_fwd(x, pf(k.n1g), pf(k.n1b), k.ln1o, k.m1, k.r1, T, C, cfg.ln_eps, stream))) return rc;
-  if ((rc = linear_fwd(k.qkv, k.ln1o, dqkv, nullptr, T))) return rc;   // dqkv doubles as the forward staging buffer
-  if ((rc = window_qkv(dqkv, k.qw, k.kw, k.vw, w, Hh, D, 0, stream))) return rc;
-  const long long hs = (long long)L * D, ws = (long long)Hh * L * D;
-  BgemmDesc sc = {L, LP, D, Hh, nWin, D, hs, ws, D, hs, ws, LP, (long long)L * LP, (long long)Hh * L * LP, scale, 0, 0};
-  if ((rc = bgemm_bf16(sc, k.qw, k.kw, k.Pm, stream))) return rc;
-  if ((rc = relbias_build(pf(k.table), relbias, Hh, WS, stream))) return rc;
-  if ((rc = window_softmax_fwd(k.Pm, relbias, w, Hh, LP, stream))) return rc;
-  if ((rc = transpose_pad(k.vw, tA, L, D, D, hs, (int64_t)nWin * Hh, LP, stream))) return rc;   // V^T [z][D][LP]
-  BgemmDesc av = {L, D, LP, Hh, nWin, LP, (long long)L * LP, (long long)Hh * L * LP, LP, (long long)D * LP,
-                  (long long)Hh * D * LP, C, D, (long long)L * C, 1.f, 0, 0};
-  if ((rc = bgemm_bf16(av, k.Pm, tA, ow, stream))) return rc;                               // [win][tok][C]
-  if ((rc = window_permute(ow, k.att, w, C, 1, stream))) return rc;
+  if (k.fused) {
+    if ((rc = linear_fwd(k.qkv, k.ln1o, k.qkv_o, nullptr, T))) return rc;
+    if ((rc = window_attention_fwd(k.qkv_o, pf(k.table), k.att, w, Hh, D, scale, stream))) return rc;
+  } else {
+    if ((rc = linear_fwd(k.qkv, k.ln1o, dqkv, nullptr, T))) return rc;   // dqkv doubles as the forward staging buffer
+    if ((rc = window_qkv(dqkv, k.qw, k.kw, k.vw, w, Hh, D, 0, stream))) return rc;
+    const long long hs = (long long)L * D, ws = (long long)Hh * L * D;
+    BgemmDesc sc = {L, LP, D, Hh, nWin, D, hs, ws, D, hs, ws, LP, (long long)L * LP, (long long)Hh * L * LP, scale, 0, 0};
+    if ((rc = bgemm_bf16(sc, k.qw, k.kw, k.Pm, stream))) return rc;
+    if ((rc = relbias_build(pf(k.table), relbias, Hh, WS, stream))) return rc;
+    if ((rc = window_softmax_fwd(k.Pm, relbias, w, Hh, LP, stream))) return rc;
+    if ((rc = transpose_pad(k.vw, tA, L, D, D, hs, (int64_t)nWin * Hh, LP, stream))) return rc;   // V^T [z][D][LP]
+    BgemmDesc av = {L, D, LP, Hh, nWin, LP, (long long)L * LP, (long long)Hh * L * LP, LP, (long long)D * LP,
+                    (long long)Hh * D * LP, C, D, (long long)L * C, 1.f, 0, 0};
+    if ((rc = bgemm_bf16(av, k.Pm, tA, ow, stream))) return rc;                               // [win][tok][C]
+    if ((rc = window_permute(ow, k.att, w, C, 1, stream))) return rc;
+  }
   if ((rc = linear_fwd(k.proj, k.att, k.x2, x, T))) return rc;
   if ((rc = layernorm_fwd(k.x2, pf(k.n2g), pf(k.n2b), k.ln2o, k.m2, k.r2, T, C, cfg.ln_eps, stream))) return rc;
   if ((rc = linear_fwd(k.fc, k.ln2o, k.h, nullptr, T))) return rc;
@@ -344,26 +358,31 @@ int Swin::block_bwd(Blk& k, const __nv_bfloat16* xin, __nv_bfloat16*& dx, __nv_b
                           stream)))
     return rc;  // dx_other: gradient w.r.t. x2
   if ((rc = linear_bwd(k.proj, dx_other, k.att, datt, T))) return rc;
-  if ((rc = window_qkv(datt, dOh, nullptr, nullptr, w, Hh, D, 0, stream))) return rc;          // dO [win][head][tok][D]
-  // dP = dO V^T
-  BgemmDesc dp = {L, LP, D, Hh, nWin, D, hs, ws, D, hs, ws, LP, ps, pws, 1.f, 0, 0};
-  if ((rc = bgemm_bf16(dp, dOh, k.vw, dP, stream))) return rc;
-  // dV = P^T dO
-  if ((rc = transpose_pad(k.Pm, tP, L, L, LP, ps, Z, LP, stream))) return rc;
-  if ((rc = transpose_pad(dOh, tA, L, D, D, hs, Z, LP, stream))) return rc;
-  BgemmDesc dv = {L, D, LP, Hh, nWin, LP, ps, pws, LP, ts, tws, D, hs, ws, 1.f, 0, 0};
-  if ((rc = bgemm_bf16(dv, tP, tA, dvw, stream))) return rc;
-  // dS, table gradient
-  if ((rc = window_softmax_bwd(k.Pm, dP, Z, L, LP, stream))) return rc;
-  if ((rc = relbias_grad(dP, dbias, gf(k.table), nWin, Hh, WS, LP, stream))) return rc;
-  // dQ = dS K * scale, dK = dS^T Q * scale
-  if ((rc = transpose_pad(k.kw, tA, L, D, D, hs, Z, LP, stream))) return rc;
-  BgemmDesc dq = {L, D, LP, Hh, nWin, LP, ps, pws, LP, ts, tws, D, hs, ws, scale, 0, 0};
-  if ((rc = bgemm_bf16(dq, dP, tA, dqw, stream))) return rc;
-  if ((rc = transpose_pad(dP, tP, L, L, LP, ps, Z, LP, stream))) return rc;
-  if ((rc = transpose_pad(k.qw, tB, L, D, D, hs, Z, LP, stream))) return rc;
-  if ((rc = bgemm_bf16(dq, tP, tB, dkw, stream))) return rc;
-  if ((rc = window_qkv(dqkv, dqw, dkw, dvw, w, Hh, D, 1, stream))) return rc;
+  if (k.fused) {
+    if ((rc = window_attention_bwd(k.qkv_o, pf(k.table), datt, dqkv, dP, LP, w, Hh, D, scale, stream))) return rc;
+    if ((rc = relbias_grad(dP, dbias, gf(k.table), nWin, Hh, WS, LP, stream))) return rc;
+  } else {
+    if ((rc = window_qkv(datt, dOh, nullptr, nullptr, w, Hh, D, 0, stream))) return rc;          // dO [win][head][tok][D]
+    // dP = dO V^T
+    BgemmDesc dp = {L, LP, D, Hh, nWin, D, hs, ws, D, hs, ws, LP, ps, pws, 1.f, 0, 0};
+    if ((rc = bgemm_bf16(dp, dOh, k.vw, dP, stream))) return rc;
+    // dV = P^T dO
+    if ((rc = transpose_pad(k.Pm, tP, L, L, LP, ps, Z, LP, stream))) return rc;
+    if ((rc = transpose_pad(dOh, tA, L, D, D, hs, Z, LP, stream))) return rc;
+    BgemmDesc dv = {L, D, LP, Hh, nWin, LP, ps, pws, LP, ts, tws, D, hs, ws, 1.f, 0, 0};
+    if ((rc = bgemm_bf16(dv, tP, tA, dvw, stream))) return rc;
+    // dS, table gradient
+    if ((rc = window_softmax_bwd(k.Pm, dP, Z, L, LP, stream))) return rc;
+    if ((rc = relbias_grad(dP, dbias, gf(k.table), nWin, Hh, WS, LP, stream))) return rc;
+    // dQ = dS K * scale, dK = dS^T Q * scale
+    if ((rc = transpose_pad(k.kw, tA, L, D, D, hs, Z, LP, stream))) return rc;
+    BgemmDesc dq = {L, D, LP, Hh, nWin, LP, ps, pws, LP, ts, tws, D, hs, ws, scale, 0, 0};
+    if ((rc = bgemm_bf16(dq, dP, tA, dqw, stream))) return rc;
+    if ((rc = transpose_pad(dP, tP, L, L, LP, ps, Z, LP, stream))) return rc;
+    if ((rc = transpose_pad(k.qw, tB, L, D, D, hs, Z, LP, stream))) return rc;
+    if ((rc = bgemm_bf16(dq, tP, tB, dkw, stream))) return rc;
+    if ((rc = window_qkv(dqkv, dqw, dkw, dvw, w, Hh, D, 1, stream))) return rc;
+  }
   if ((rc = linear_bwd(k.qkv, dqkv, k.ln1o, dln, T))) return rc;
   if ((rc = join_side())) return rc;  // the next kernel overwrites dx, which this block's first weight gradient read
   return layernorm_bwd(dln, xin, pf(k.n1g), k.m1, k.r1, dx_other, dx, gf(k.n1g), gf(k.n1b), T, C, scratch, scratch_bytes,

@@ -7,6 +7,7 @@
 // for the column reductions.
 #include "common.cuh"
 #include "ops.cuh"
+#include "window_geom.cuh"
 
 namespace srt {
 
@@ -714,22 +715,6 @@ gelu_erf_bwd_kernel(const bf16* __restrict__ dy, const bf16* __restrict__ x, bf1
 }
 
 // ---- shifted-window attention helpers (Swin) ------------------------------------------------------------
-// Tokens live in the natural [B][Hs][Ws] order. A window of WS x WS tokens of the cyclically shifted map is
-// window (wy, wx), token (iy, ix): shifted position (wy*WS+iy, wx*WS+ix), natural position that plus `shift`
-// modulo the map size.
-struct WinGeom {
-  int B, Hs, Ws, WS, shift, nWy, nWx;
-};
-__device__ inline int64_t win_token_to_natural(const WinGeom& g, int64_t win, int tok) {
-  const int wx = (int)(win % g.nWx);
-  const int wy = (int)((win / g.nWx) % g.nWy);
-  const int64_t b = win / ((int64_t)g.nWx * g.nWy);
-  const int iy = tok / g.WS, ix = tok - iy * g.WS;
-  int h = wy * g.WS + iy + g.shift, w = wx * g.WS + ix + g.shift;
-  if (h >= g.Hs) h -= g.Hs;
-  if (w >= g.Ws) w -= g.Ws;
-  return (b * g.Hs + h) * g.Ws + w;
-}
 // dir 0: out_win[win][tok][c] = in_nat[natural][c]; dir 1: out_nat[natural][c] = in_win[win][tok][c]. C % 8 == 0.
 __global__ void __launch_bounds__(NT)
 window_permute_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, WinGeom g, int C, int dir) {
@@ -781,9 +766,6 @@ relbias_build_kernel(const float* __restrict__ table, float* __restrict__ relbia
     const int j = i % L, r = (i / L) % L, hd = i / (L * L);
     relbias[i] = table[relpos_index(r, j, WS) * heads + hd];
   }
-}
-__device__ inline int shift_region(int p, int size, int WS, int shift) {  // region of a shifted coordinate
-  return p < size - WS ? 0 : (p < size - shift ? 1 : 2);
 }
 // scores [Z][L][ld] (Z = windows * heads, head fastest): P = softmax(scores + relbias + mask) over the L valid
 // columns, columns L..ld-1 are written as zero. One warp per row.

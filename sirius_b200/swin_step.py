@@ -20,6 +20,8 @@ class SwinConfigC(C.Structure):
 
 
 register({
+    "srt_window_attention_fwd": (None, [_vp, _vp, _vp] + [_i] * 7 + [C.c_float, _vp]),
+    "srt_window_attention_bwd": (None, [_vp] * 5 + [_i] * 8 + [C.c_float, _vp]),
     "srt_swin_create": (None, [C.POINTER(SwinConfigC), C.POINTER(_vp)]),
     "srt_swin_destroy": (None, [_vp]),
     "srt_swin_num_params": (_i, [_vp]),
