@@ -70,6 +70,8 @@ int srt_conv_wgrad(const srt_conv_desc* d, int dtype, int impl, const void* dy, 
                    float* dw, void* scratch, size_t scratch_bytes, void* stream);
 size_t srt_conv_wgrad_scratch_bytes(const srt_conv_desc* d, int dtype, int impl);
 /* wt[C,R,S,K] = transpose of w[K,R,S,C] (same dtype). */
+int srt_conv_dgrad_direct(const srt_conv_desc* d, int dtype, int impl, const void* dy, const void* w, void* dx,
+                          const srt_conv_epilogue* ep, void* stream); /* w[K,R,S,C] itself; bf16, stride 1, K % 64 == 0 or 1x1 */
 int srt_conv_filter_transpose(const srt_conv_desc* d, int dtype, const void* w, void* wt,
                               void* stream);
 

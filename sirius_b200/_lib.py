@@ -44,6 +44,7 @@ _SIGNATURES = {
     "srt_last_error": (C.c_char_p, []),
     "srt_version": (C.c_char_p, []),
     "srt_conv_fprop": (None, [_PD, _i, _i, _vp, _vp, _vp, _PE, _vp]),
+    "srt_conv_dgrad_direct": (None, [_PD, _i, _i, _vp, _vp, _vp, _PE, _vp]),
     "srt_conv_fprop_infer": (None, [_PD, _i, _i, _vp, _vp, _vp, _vp, _vp, _vp, _i, _vp]),
     "srt_conv_fprop_bn_stats": (None, [_PD, _i, _i, _vp, _vp, _vp, _PE, _vp, _sz, C.POINTER(C.c_int), _vp]),
     "srt_conv_fprop_bn_stats_bytes": (_sz, [_PD]),

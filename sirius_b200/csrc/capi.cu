@@ -158,6 +158,15 @@ int conv_dgrad(const srt_conv_desc& d, int dtype, int impl, const void* dy, cons
   return conv_gather_gemm_simt(g, dtype, dy, wt, dx, ep, st);
 }
 
+bool conv_dgrad_direct_supported(const srt_conv_desc& d, int dtype, int impl) { return use_tc(dtype, impl) && conv_dgrad_direct_ok(d); }
+int conv_dgrad_direct(const srt_conv_desc& d, int dtype, int impl, const void* dy, const void* w, void* dx,
+                      const srt_conv_epilogue* ep, cudaStream_t st) {
+  int rc = check_desc(d);
+  if (rc) return rc;
+  SRT_REQUIRE(conv_dgrad_direct_supported(d, dtype, impl), "conv: this data gradient needs the transposed filter");
+  return conv_dgrad_direct_tc(make_dgrad_geom(d), dy, w, dx, ep, st);
+}
+
 size_t conv_wgrad_scratch_bytes(const srt_conv_desc& d, int dtype, int impl) {
   GatherGeom g = make_fprop_geom(d);
   return use_tc(dtype, impl) ? conv_wgrad_tc_scratch_bytes(g) : conv_wgrad_simt_scratch_bytes(g);
@@ -208,6 +217,12 @@ int srt_conv_fprop_bn_stats(const srt_conv_desc* d, int dtype, int impl, const v
 size_t srt_conv_fprop_bn_stats_bytes(const srt_conv_desc* d) { return d ? conv_fprop_stats_bytes(*d) : 0; }
 int srt_conv_fprop_bn_stats_supported(const srt_conv_desc* d, int dtype, int impl) {
   return d && conv_fprop_stats_supported(*d, dtype, impl) ? 1 : 0;
+}
+int srt_conv_dgrad_direct(const srt_conv_desc* d, int dtype, int impl, const void* dy, const void* w, void* dx,
+                          const srt_conv_epilogue* ep, void* stream) {
+  SRT_REQUIRE(d && dy && w && dx, "conv_dgrad_direct: null argument");
+  CHECK_DTYPE(dtype);
+  return conv_dgrad_direct(*d, dtype, impl, dy, w, dx, ep, (cudaStream_t)stream);
 }
 int srt_conv_dgrad(const srt_conv_desc* d, int dtype, int impl, const void* dy, const void* wt,
                    void* dx, const srt_conv_epilogue* ep, void* stream) {

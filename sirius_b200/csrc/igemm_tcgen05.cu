@@ -535,6 +535,10 @@ struct PersistParams {
   int im_stride;
   int im_cpt;            // im2col: 64-channel chunks per filter tap (k-block kb = tap * im_cpt + chunk)
   int im_flip;           // im2col: taps run backwards (data gradient)
+  // Data gradient on the filter as the forward pass stores it, [reduction channel][tap][Nout]: the B tile of a k-block is
+  // 64 reduction rows of BN output columns, an MN-major operand (one 64 x 64 block after the other), and no transposed copy
+  // of the weights is kept or refreshed. 0: B is [Nout][Kg], K-major.
+  int b_mn;
   int m_tiles, n_tiles;  // 128-row tiles and BN-column tiles of the output
   int gather_lag;        // cp.async groups a gather thread keeps in flight before it hands a stage over (1..NS-2)
   int* status;
@@ -688,19 +692,33 @@ igemm_fwd_persistent(const PersistParams p, const __grid_constant__ CUtensorMap 
           if (PAIR) {
             const uint32_t lbar = map_to_cta(smem_u32(&full[s]), 0u);
             if (rank == 0) mbar_arrive_expect_tx(smem_u32(&full[s]), bytes);
-            tma_load_2d_pair(smem_u32(sB + s * B_STAGE_BYTES), &tmap_b, lbar, kb * BK, n0);
+            if (p.b_mn) {
+#pragma unroll
+              for (int blk = 0; blk < B_ROWS / 64; ++blk)
+                tma_load_2d_pair(smem_u32(sB + s * B_STAGE_BYTES) + (uint32_t)blk * 8192u, &tmap_b, lbar,
+                                 (tap_r * g.S + tap_s) * g.Nout + n0 + blk * 64, chunk * BK);
+            } else {
+              tma_load_2d_pair(smem_u32(sB + s * B_STAGE_BYTES), &tmap_b, lbar, kb * BK, n0);
+            }
             if (p.a_tma == 1) tma_load_2d_pair(smem_u32(sA + s * A_STAGE_BYTES), &tmap_a, lbar, kb * BK, m0);
             else if (p.a_tma == 2)
               tma_load_im2col_4d_pair(smem_u32(sA + s * A_STAGE_BYTES), &tmap_a, lbar, chunk * BK, iw0, ih0, in0, off_w, off_h);
           } else {
             const uint32_t bar = smem_u32(&full[s]);
             mbar_arrive_expect_tx(bar, bytes);
-            tma_load_2d(smem_u32(sB + s * B_STAGE_BYTES), &tmap_b, bar, kb * BK, n0);
+            if (p.b_mn) {
+#pragma unroll
+              for (int blk = 0; blk < B_ROWS / 64; ++blk)
+                tma_load_2d(smem_u32(sB + s * B_STAGE_BYTES) + (uint32_t)blk * 8192u, &tmap_b, bar,
+                            (tap_r * g.S + tap_s) * g.Nout + n0 + blk * 64, chunk * BK);
+            } else {
+              tma_load_2d(smem_u32(sB + s * B_STAGE_BYTES), &tmap_b, bar, kb * BK, n0);
+            }
             if (p.a_tma == 1) tma_load_2d(smem_u32(sA + s * A_STAGE_BYTES), &tmap_a, bar, kb * BK, m0);
             else if (p.a_tma == 2)
               tma_load_im2col_4d(smem_u32(sA + s * A_STAGE_BYTES), &tmap_a, bar, chunk * BK, iw0, ih0, in0, off_w, off_h);
           }
-          if (p.a_tma == 2 && ++chunk == p.im_cpt) {
+          if (++chunk == p.im_cpt) {
             chunk = 0;
             if (++tap_s == g.S) { tap_s = 0; ++tap_r; }
           }
@@ -710,7 +728,9 @@ igemm_fwd_persistent(const PersistParams p, const __grid_constant__ CUtensorMap 
   } else if (warp == 1) {
     // ---------------- MMA issuer (the leader's, in a pair) ----------------
     if (lane == 0 && rank == 0) {
-      constexpr uint32_t idesc = make_idesc_bf16(BM * NCTA, BN, 0, 0);
+      const uint32_t idesc = p.b_mn ? make_idesc_bf16(BM * NCTA, BN, 0, 1) : make_idesc_bf16(BM * NCTA, BN, 0, 0);
+      // 16 reduction elements further: two groups of eight rows of the MN-major tile, or 32 bytes of every K-major row
+      const uint32_t b_step = p.b_mn ? 2048u : 32u, b_lbo = p.b_mn ? 8192u : 0u;
       int it = 0, tc = 0;
       bool ok = true;
       for (int t = unit; t < total_tiles && ok; t += nunits, ++tc) {
@@ -734,7 +754,7 @@ igemm_fwd_persistent(const PersistParams p, const __grid_constant__ CUtensorMap 
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
             const uint64_t ad = make_smem_desc_sw128(a0 + k * 32, 0, 1024);
-            const uint64_t bd = make_smem_desc_sw128(b0 + k * 32, 0, 1024);
+            const uint64_t bd = make_smem_desc_sw128(b0 + k * b_step, b_lbo, 1024);
             if (PAIR) umma_bf16_pair(acc, ad, bd, idesc, (kb | k) != 0 ? 1u : 0u);
             else umma_bf16(acc, ad, bd, idesc, (kb | k) != 0 ? 1u : 0u);
           }
@@ -1786,8 +1806,9 @@ void tc_set_conv_plan(int gather, int tile_n, int pair) {
 template <bool INFER>
 static int conv_gather_gemm_tc_persistent(const GatherGeom& g, const void* src, const void* Bm, void* D,
                                           const srt_conv_epilogue* ep, cudaStream_t st, double* col_partial = nullptr,
-                                          const InferEpilogue* infer = nullptr) {
+                                          const InferEpilogue* infer = nullptr, bool b_mn = false) {
   PersistParams p;
+  p.b_mn = b_mn;
   p.scale = infer ? infer->scale : nullptr;
   p.act = infer ? infer->act : ACT_NONE;
   p.g = g;
@@ -1802,11 +1823,11 @@ static int conv_gather_gemm_tc_persistent(const GatherGeom& g, const void* src, 
   const bool plain = g.R == 1 && g.S == 1 && g.stride == 1 && g.pad == 0;
   p.a_tma = g_force_gather ? 0 : plain ? 1 : (im2col_ok(g) && g_im2col_enabled) ? 2 : 0;
   p.im_lower_w = p.im_lower_h = p.im_flip = 0;
-  p.im_stride = p.im_cpt = 1;
+  p.im_stride = 1;
+  p.im_cpt = ceil_div(g.src_c, BK);
   if (p.a_tma == 2) {
     const Im2colBox b = im2col_box(g);
     p.im_lower_w = b.lower_w; p.im_lower_h = b.lower_h; p.im_stride = b.stride;
-    p.im_cpt = g.src_c / BK;
     p.im_flip = g.dgrad;
   }
   p.gather_lag = 0;  // set with the stage count below
@@ -1828,7 +1849,8 @@ static int conv_gather_gemm_tc_persistent(const GatherGeom& g, const void* src, 
   p.m_tiles = ceil_div(g.M, BM);
   p.n_tiles = ceil_div(g.Nout, bn);
   CUtensorMap tb, ta, td;
-  int rc = make_tmap_2d(&tb, Bm, (uint64_t)g.Nout, (uint64_t)g.Kg, (uint32_t)(pair ? bn / 2 : bn));
+  int rc = b_mn ? make_tmap_2d(&tb, Bm, (uint64_t)g.src_c, (uint64_t)g.R * g.S * g.Nout, 64)
+                : make_tmap_2d(&tb, Bm, (uint64_t)g.Nout, (uint64_t)g.Kg, (uint32_t)(pair ? bn / 2 : bn));
   if (rc != SRT_OK) return rc;
   if (p.a_tma == 1) {
     rc = make_tmap_2d(&ta, src, (uint64_t)g.M, (uint64_t)g.Kg, (uint32_t)BM);
@@ -1864,6 +1886,16 @@ int conv_gather_gemm_tc(const GatherGeom& g, const void* src, const void* Bm, vo
               "tcgen05 conv: channel counts (%d, %d) must be multiples of 8", g.src_c, g.Nout);
   SRT_REQUIRE(((uintptr_t)src & 15) == 0 && ((uintptr_t)D & 15) == 0, "tcgen05 conv: unaligned tensor");
   return conv_gather_gemm_tc_persistent<false>(g, src, Bm, D, ep, st);
+}
+
+// Data gradient on the filter w[K][R][S][C] itself: a k-block must lie inside one filter tap, and the walk over output
+// positions must be that of a stride-1 filter.
+bool conv_dgrad_direct_ok(const srt_conv_desc& d) {
+  return d.stride == 1 && d.C % 8 == 0 && d.K % 8 == 0 && (d.K % BK == 0 || d.R * d.S == 1);
+}
+int conv_dgrad_direct_tc(const GatherGeom& g, const void* dy, const void* w, void* dx, const srt_conv_epilogue* ep, cudaStream_t st) {
+  SRT_REQUIRE(((uintptr_t)dy & 15) == 0 && ((uintptr_t)dx & 15) == 0, "tcgen05 conv: unaligned tensor");
+  return conv_gather_gemm_tc_persistent<false>(g, dy, w, dx, ep, st, nullptr, nullptr, true);
 }
 
 // Cluster size of the split kernel, 1 where the persistent kernel is the better one: the tiles times the cluster must fit

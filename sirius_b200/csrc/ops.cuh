@@ -79,6 +79,10 @@ int conv_fprop_infer(const srt_conv_desc& d, int dtype, int impl, const void* x,
                      cudaStream_t st);
 int conv_dgrad(const srt_conv_desc& d, int dtype, int impl, const void* dy, const void* wt,
                void* dx, const srt_conv_epilogue* ep, cudaStream_t st);
+// The same gradient on the filter w itself, without a transposed copy (bf16 tensor-core path, see conv_dgrad_direct_ok).
+bool conv_dgrad_direct_supported(const srt_conv_desc& d, int dtype, int impl);
+int conv_dgrad_direct(const srt_conv_desc& d, int dtype, int impl, const void* dy, const void* w, void* dx,
+                      const srt_conv_epilogue* ep, cudaStream_t st);
 // fprop that also leaves the column sums of y for bn_finalize (bf16 tensor-core path only; ask
 // conv_fprop_stats_supported first). `partial` needs conv_fprop_stats_bytes(d) bytes; *slabs receives the number
 // of partial rows written.

@@ -39,10 +39,10 @@ struct Gpt2 {
   std::vector<Rec> params;
   size_t n_flat = 0;
   float *P = nullptr, *G = nullptr, *M1 = nullptr, *M2 = nullptr;
-  __nv_bfloat16 *Pw = nullptr, *WT = nullptr;  // bf16 copy; per-linear transposes [in][out] for the data gradients
+  __nv_bfloat16* Pw = nullptr;  // bf16 copy
   int opt_steps = 0;
 
-  struct Lin { int w, b, in, out; size_t wt_off; };
+  struct Lin { int w, b, in, out; };
   struct Layer {
     int ln1_g, ln1_b, ln2_g, ln2_b;
     Lin qkv, proj, fc, fc2;
@@ -53,7 +53,6 @@ struct Gpt2 {
   };
   std::vector<Layer> layers;
   int wte, wpe, lnf_g, lnf_b;
-  size_t wte_wt_off = 0, n_wt = 0;
 
   // activations / scratch
   __nv_bfloat16 *x0 = nullptr, *lnfo = nullptr, *logits = nullptr;
@@ -189,8 +188,6 @@ struct Gpt2 {
     l.in = in; l.out = out;
     l.w = add(pre + ".weight", in, out, 1, (size_t)in * out);
     l.b = add(pre + ".bias", out, 0, 0, (size_t)out);
-    l.wt_off = n_wt;
-    n_wt += up((size_t)in * out, 64);
     return l;
   }
   float* pf(int i) { return P + params[i].off; }
@@ -226,7 +223,7 @@ struct Gpt2 {
       if ((rc = conv_wgrad(lin_desc(T, l.in, l.out), SRT_BF16, SRT_IMPL_AUTO, dy, x, gf(l.w), wscratch, scratch_bytes, ws)))
         return rc;
     }
-    if (dx) return conv_dgrad(lin_desc(T, l.in, l.out), SRT_BF16, SRT_IMPL_AUTO, dy, WT + l.wt_off, dx, nullptr, stream);
+    if (dx) return conv_dgrad_direct(lin_desc(T, l.in, l.out), SRT_BF16, SRT_IMPL_AUTO, dy, pw(l.w), dx, nullptr, stream);
     return SRT_OK;
   }
 };
@@ -256,8 +253,6 @@ int Gpt2::build() {
   }
   lnf_g = add("transformer.ln_f.weight", C, 0, 0, C);
   lnf_b = add("transformer.ln_f.bias", C, 0, 0, C);
-  wte_wt_off = n_wt;
-  n_wt += up((size_t)Vpad * C, 64);
 
   int rc;
   if ((rc = dalloc(&P, n_flat * 4, true))) return rc;
@@ -265,7 +260,6 @@ int Gpt2::build() {
   if ((rc = dalloc(&M1, n_flat * 4, true))) return rc;
   if ((rc = dalloc(&M2, n_flat * 4, true))) return rc;
   if ((rc = dalloc(&Pw, n_flat * 2, true))) return rc;
-  if ((rc = dalloc(&WT, n_wt * 2, true))) return rc;
 
   if ((rc = dalloc(&ACC, n_flat * 4, true))) return rc;
   // scratch: split partials of the largest filter gradient, norm / bias column partials (sized for max_batch)
@@ -330,15 +324,8 @@ int Gpt2::alloc_activations(int B) {
   return SRT_OK;
 }
 
-// bf16 working copy and the transposed weights the data gradients read.
-int Gpt2::refresh() {
-  int rc;
-  if ((rc = cast_f32_to_bf16(P, Pw, (int64_t)n_flat, stream))) return rc;
-  auto tr = [&](const Lin& l) { return filter_transpose(SRT_BF16, pw(l.w), WT + l.wt_off, l.out, 1, l.in, stream); };
-  for (Layer& y : layers)
-    if ((rc = tr(y.qkv)) || (rc = tr(y.proj)) || (rc = tr(y.fc)) || (rc = tr(y.fc2))) return rc;
-  return filter_transpose(SRT_BF16, pw(wte), WT + wte_wt_off, Vpad, 1, C, stream);
-}
+// bf16 working copy.
+int Gpt2::refresh() { return cast_f32_to_bf16(P, Pw, (int64_t)n_flat, stream); }
 
 // Causal attention of one layer: qkv_o -> att. 64-channel heads take the fused kernel; other sizes go through the
 // score matrix.
@@ -435,7 +422,7 @@ int Gpt2::backward(int B, int global_batch) {
                               stream))) {
     return rc;
   }
-  if ((rc = conv_dgrad(lin_desc(T, C, Vpad), SRT_BF16, SRT_IMPL_AUTO, logits, WT + wte_wt_off, dln, nullptr, stream))) return rc;
+  if ((rc = conv_dgrad_direct(lin_desc(T, C, Vpad), SRT_BF16, SRT_IMPL_AUTO, logits, pw(wte), dln, nullptr, stream))) return rc;
   const __nv_bfloat16* x_last = L > 0 ? layers[L - 1].xout : x0;
   if ((rc = layernorm_bwd(dln, x_last, pf(lnf_g), lnf_mean, lnf_rstd, nullptr, dxa, gf(lnf_g), gf(lnf_b), T, C, scratch,
                           scratch_bytes, stream)))
@@ -613,12 +600,7 @@ int srt_gpt2_optimizer(srt_gpt2* h) {
     SRT_CHECK_CUDA(cudaMemsetAsync(g->ACC, 0, g->n_flat * 4, g->stream));
     g->accum_pending = 0;
   }
-  auto tr = [&](const Gpt2::Lin& l) {
-    return filter_transpose(SRT_BF16, g->pw(l.w), g->WT + l.wt_off, l.out, 1, l.in, g->stream);
-  };
-  for (Gpt2::Layer& y : g->layers)
-    if ((rc = tr(y.qkv)) || (rc = tr(y.proj)) || (rc = tr(y.fc)) || (rc = tr(y.fc2))) return rc;
-  return filter_transpose(SRT_BF16, g->pw(g->wte), g->WT + g->wte_wt_off, g->Vpad, 1, g->C, g->stream);
+  return SRT_OK;
 }
 
 // Mean next-token loss of the last micro-batch over its own targets (what the reference's model returns).

@@ -36,12 +36,12 @@ struct Qwen2 {
 
   struct Rec { std::string name; size_t off, count; int64_t shape[2]; int ndim; };
   std::vector<Rec> params;
-  size_t n_flat = 0, n_wt = 0;
+  size_t n_flat = 0;
   float *P = nullptr, *G = nullptr, *M1 = nullptr, *M2 = nullptr;
-  __nv_bfloat16 *Pw = nullptr, *WT = nullptr;
+  __nv_bfloat16* Pw = nullptr;
   int opt_steps = 0;
 
-  struct Lin { size_t w_off; long long b_off; int in, out; size_t wt_off; };  // offsets into the flat buffers; b_off < 0 = no bias
+  struct Lin { size_t w_off; long long b_off; int in, out; };  // offsets into the flat buffers; b_off < 0 = no bias
   struct Layer {
     int n1, n2;
     Lin qkv, o, gu, down;
@@ -51,7 +51,6 @@ struct Qwen2 {
   };
   std::vector<Layer> layers;
   int emb, nf;
-  size_t emb_wt_off = 0;
 
   __nv_bfloat16 *x0 = nullptr, *nfo = nullptr, *logits = nullptr;
   float *zf = nullptr, *rf = nullptr, *row_loss = nullptr, *loss_acc = nullptr;
@@ -184,15 +183,13 @@ struct Qwen2 {
     return (int)params.size() - 1;
   }
   Lin make_lin(size_t w_off, long long b_off, int in, int out) {
-    Lin l = {w_off, b_off, in, out, n_wt};
-    n_wt += upq((size_t)in * out, 64);
+    Lin l = {w_off, b_off, in, out};
     return l;
   }
   float* pf(int i) { return P + params[i].off; }
   float* gf(int i) { return G + params[i].off; }
 
   int build();
-  int transposes();
   int attention_forward(Layer& y, int B, float scale);
   int attention_backward(Layer& y, int B, float scale);
   int forward(int B);
@@ -219,7 +216,7 @@ struct Qwen2 {
       if ((rc = conv_wgrad(lin_desc(T, l.in, l.out), SRT_BF16, SRT_IMPL_AUTO, dy, x, G + l.w_off, wscratch, scratch_bytes, ws)))
         return rc;
     }
-    if (dx) return conv_dgrad(lin_desc(T, l.in, l.out), SRT_BF16, SRT_IMPL_AUTO, dy, WT + l.wt_off, dx, nullptr, stream);
+    if (dx) return conv_dgrad_direct(lin_desc(T, l.in, l.out), SRT_BF16, SRT_IMPL_AUTO, dy, Pw + l.w_off, dx, nullptr, stream);
     return SRT_OK;
   }
 };
@@ -259,12 +256,10 @@ int Qwen2::build() {
     y.down = make_lin(params[dw].off, -1, F, C);
   }
   nf = add("model.norm.weight", C, 0, C);
-  emb_wt_off = n_wt;
-  n_wt += upq((size_t)Vpad * C, 64);
 
   int rc;
   if ((rc = dalloc(&P, n_flat * 4, true)) || (rc = dalloc(&G, n_flat * 4, true)) || (rc = dalloc(&M1, n_flat * 4, true)) ||
-      (rc = dalloc(&M2, n_flat * 4, true)) || (rc = dalloc(&Pw, n_flat * 2, true)) || (rc = dalloc(&WT, n_wt * 2, true)))
+      (rc = dalloc(&M2, n_flat * 4, true)) || (rc = dalloc(&Pw, n_flat * 2, true)))
     return rc;
   if ((rc = dalloc(&ACC, n_flat * 4, true)) || (rc = dalloc(&loss_acc, 256, true))) return rc;
   const size_t T = (size_t)cfg.max_batch * S;
@@ -331,14 +326,6 @@ int Qwen2::alloc_activations(int B) {
     return rc;
   act_batch = B;
   return SRT_OK;
-}
-
-int Qwen2::transposes() {
-  int rc;
-  auto tr = [&](const Lin& l) { return filter_transpose(SRT_BF16, Pw + l.w_off, WT + l.wt_off, l.out, 1, l.in, stream); };
-  for (Layer& y : layers)
-    if ((rc = tr(y.qkv)) || (rc = tr(y.o)) || (rc = tr(y.gu)) || (rc = tr(y.down))) return rc;
-  return filter_transpose(SRT_BF16, Pw + params[emb].off, WT + emb_wt_off, Vpad, 1, C, stream);
 }
 
 // Causal grouped-query attention of one layer: qkv_o (rotated) -> att. 64-channel heads take the fused kernel; other
@@ -439,7 +426,7 @@ int Qwen2::backward(int B, int global_batch) {
                               stream))) {
     return rc;
   }
-  if ((rc = conv_dgrad(lin_desc(T, C, Vpad), SRT_BF16, SRT_IMPL_AUTO, logits, WT + emb_wt_off, dln, nullptr, stream))) return rc;
+  if ((rc = conv_dgrad_direct(lin_desc(T, C, Vpad), SRT_BF16, SRT_IMPL_AUTO, logits, Pw + params[emb].off, dln, nullptr, stream))) return rc;
   const __nv_bfloat16* x_last = L > 0 ? layers[L - 1].xout : x0;
   if ((rc = rmsnorm_bwd(dln, x_last, pf(nf), zf, rf, nullptr, dxa, gf(nf), T, C, scratch, scratch_bytes, stream))) return rc;
   __nv_bfloat16 *dx = dxa, *dx_other = dxb;
@@ -535,7 +522,6 @@ int srt_qwen2_commit_params(srt_qwen2* h) {
   Qwen2* g = (Qwen2*)h;
   SRT_REQUIRE(g, "qwen2_commit_params: null handle");
   int rc = cast_f32_to_bf16(g->P, g->Pw, (int64_t)g->n_flat, g->stream);
-  if (rc == SRT_OK) rc = g->transposes();
   if (rc) return rc;
   SRT_CHECK_CUDA(cudaStreamSynchronize(g->stream));
   return SRT_OK;
@@ -597,7 +583,7 @@ int srt_qwen2_optimizer(srt_qwen2* h) {
     SRT_CHECK_CUDA(cudaMemsetAsync(g->ACC, 0, g->n_flat * 4, g->stream));
     g->accum_pending = 0;
   }
-  return g->transposes();
+  return SRT_OK;
 }
 
 int srt_qwen2_loss(srt_qwen2* h, float* host_loss) {

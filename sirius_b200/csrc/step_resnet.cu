@@ -357,13 +357,20 @@ struct Step {
     params.push_back(r);
     return (int)params.size() - 1;
   }
+  // Whether the data gradient reads the filter itself: no transposed copy is kept then.
+  bool direct_dgrad(const ConvL& c) const {
+    const srt_conv_desc d = {1, 32, 32, c.C, c.K, c.R, c.S, c.stride, c.pad, 32, 32};
+    return conv_dgrad_direct_supported(d, cfg.dtype, cfg.impl);
+  }
+  bool direct_fc() const { return conv_dgrad_direct_supported({1, 1, 1, feat_C, cfg.num_classes, 1, 1, 1, 0, 1, 1}, cfg.dtype, cfg.impl); }
+  size_t fc_wt_off() const { return n_wt - align_up((size_t)cfg.num_classes * feat_C, 64); }  // stored after the conv filters
   ConvL make_conv(const std::string& name, int Cin_real, int K, int R, int stride, int pad) {
     ConvL c;
     c.C = Cin_real < 8 ? kStemCpad : Cin_real;
     c.K = K; c.R = R; c.S = R; c.stride = stride; c.pad = pad;
     c.w = add_param(name + ".weight", SRT_PARAM_CONV, {K, Cin_real, R, R}, c.C);
     c.wt_off = n_wt;
-    n_wt += align_up((size_t)K * R * R * c.C, 64);
+    if (!direct_dgrad(c)) n_wt += align_up((size_t)K * R * R * c.C, 64);
     c.s2_off = n_wt;
     if (stride == 2 && R == 3) n_wt += align_up((size_t)K * R * R * c.C, 64);  // taps regrouped by output parity
     return c;
@@ -437,9 +444,7 @@ int Step::build() {
   final_HW = H * H;
   fc_w = add_param("fc.weight", SRT_PARAM_LINEAR, {cfg.num_classes, feat_C}, 0);
   fc_b = add_param("fc.bias", SRT_PARAM_VECTOR, {cfg.num_classes}, 0);
-  const size_t fc_wt_off = n_wt;
-  n_wt += align_up((size_t)cfg.num_classes * feat_C, 64);
-  (void)fc_wt_off;
+  if (!direct_fc()) n_wt += align_up((size_t)cfg.num_classes * feat_C, 64);
   SRT_REQUIRE(cfg.num_classes % 8 == 0, "resnet: num_classes must be a multiple of 8");
 
   // ---- device memory ----
@@ -760,6 +765,7 @@ int Step::refresh_working_copies() {
   if ((rc = join_side())) return rc;
   if (cfg.dtype == SRT_BF16 && (rc = cast_f32_to_bf16(P, Pw, (int64_t)n_flat, stream))) return rc;
   auto tr = [&](const ConvL& c) -> int {
+    if (direct_dgrad(c)) return SRT_OK;
     int r = filter_transpose(cfg.dtype, pw(c.w), wt(c), c.K, c.R * c.S, c.C, stream);
     return r ? r : build_subfilters(c, stream);
   };
@@ -770,9 +776,9 @@ int Step::refresh_working_copies() {
     if ((rc = tr(k.u3.conv))) return rc;
     if (k.has_ds && (rc = tr(k.ds.conv))) return rc;
   }
-  // fc: [classes][feat] -> [feat][classes], stored after the conv filters
-  const size_t fc_wt_off = n_wt - align_up((size_t)cfg.num_classes * feat_C, 64);
-  return filter_transpose(cfg.dtype, pw(fc_w), (char*)WT + fc_wt_off * esz, cfg.num_classes, 1, feat_C, stream);
+  if (direct_fc()) return SRT_OK;
+  // fc: [classes][feat] -> [feat][classes]
+  return filter_transpose(cfg.dtype, pw(fc_w), (char*)WT + fc_wt_off() * esz, cfg.num_classes, 1, feat_C, stream);
 }
 
 int Step::forward(int B) {
@@ -885,9 +891,9 @@ int Step::backward(int B) {
   if ((rc = timed(SRT_PROF_OTHER, (double)B * cfg.num_classes * esz, [&] {
         return colsum(dt, dlogits, B, cfg.num_classes, gf(fc_b), stream); })))
     return rc;
-  const size_t fc_wt_off = n_wt - align_up((size_t)cfg.num_classes * feat_C, 64);
   if ((rc = timed(SRT_PROF_CONV, fc_flops, [&] {
-        return conv_dgrad(fd, dt, impl, dlogits, (char*)WT + fc_wt_off * esz, T[1], nullptr, stream); })))
+        return direct_fc() ? conv_dgrad_direct(fd, dt, impl, dlogits, pw(fc_w), T[1], nullptr, stream)
+                           : conv_dgrad(fd, dt, impl, dlogits, (char*)WT + fc_wt_off() * esz, T[1], nullptr, stream); })))
     return rc;
   if ((rc = timed(SRT_PROF_OTHER, (double)B * (final_HW + 1) * feat_C * esz, [&] {
         return avgpool_bwd(dt, T[1], T[0], B, final_HW, feat_C, stream); })))
@@ -947,6 +953,7 @@ int Step::backward(int B) {
     if (s2_fast(u.conv) && u.H % 2 == 0 && u.W % 2 == 0)
       return timed(SRT_PROF_CONV, flops, [&] { return dgrad_s2(u, dz, dx, addend, B); });
     return timed(SRT_PROF_CONV, flops, [&] {
+      if (direct_dgrad(u.conv)) return conv_dgrad_direct(d, dt, impl, dz, pw(u.conv.w), dx, addend ? &ep : nullptr, stream);
       return conv_dgrad(d, dt, impl, dz, wt(u.conv), dx, addend ? &ep : nullptr, stream); });
   };
 
@@ -1237,6 +1244,7 @@ int srt_step_optimizer(srt_step* h) {
   }
   PdlOff no_early_launch(ts != s->stream);
   auto tr = [&](const ConvL& c) -> int {
+    if (s->direct_dgrad(c)) return SRT_OK;
     int r;
     if (ts != s->stream) r = filter_transpose(s->cfg.dtype, s->pw(c.w), s->wt(c), c.K, c.R * c.S, c.C, ts);
     else r = s->timed(SRT_PROF_OPTIM, 2.0 * c.K * c.R * c.S * c.C * s->esz, [&] {
@@ -1250,8 +1258,8 @@ int srt_step_optimizer(srt_step* h) {
     if ((rc = tr(k.u3.conv))) return rc;
     if (k.has_ds && (rc = tr(k.ds.conv))) return rc;
   }
-  const size_t fc_wt_off = s->n_wt - align_up((size_t)s->cfg.num_classes * s->feat_C, 64);
-  return filter_transpose(s->cfg.dtype, s->pw(s->fc_w), (char*)s->WT + fc_wt_off * s->esz, s->cfg.num_classes, 1,
+  if (s->direct_fc()) return SRT_OK;
+  return filter_transpose(s->cfg.dtype, s->pw(s->fc_w), (char*)s->WT + s->fc_wt_off() * s->esz, s->cfg.num_classes, 1,
                           s->feat_C, ts);
 }
 

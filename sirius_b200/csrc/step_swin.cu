@@ -33,12 +33,12 @@ struct Swin {
 
   struct Rec { std::string name; size_t off, count; int64_t shape[4]; int ndim; int kind; int cpad; };  // kind 2 = conv KCRS outside
   std::vector<Rec> params;
-  size_t n_flat = 0, n_wt = 0;
+  size_t n_flat = 0;
   float *P = nullptr, *G = nullptr, *M1 = nullptr, *M2 = nullptr;
-  __nv_bfloat16 *Pw = nullptr, *WT = nullptr;
+  __nv_bfloat16* Pw = nullptr;
   int opt_steps = 0;
 
-  struct Lin { int w, b, in, out; size_t wt_off; };
+  struct Lin { int w, b, in, out; };
   struct Blk {
     int C, heads, D, Hs, shift;
     int n1g, n1b, n2g, n2b, table;
@@ -125,8 +125,6 @@ struct Swin {
     l.in = in; l.out = out;
     l.w = add(pre + ".weight", {out, in}, 0, (size_t)in * out);
     l.b = bias ? add(pre + ".bias", {out}, 0, (size_t)out) : -1;
-    l.wt_off = n_wt;
-    n_wt += up_((size_t)in * out, 64);
     return l;
   }
   float* pf(int i) { return P + params[i].off; }
@@ -154,7 +152,7 @@ struct Swin {
       if ((rc = conv_wgrad(lin_desc(T, l.in, l.out), SRT_BF16, SRT_IMPL_AUTO, dy, x, gf(l.w), wscratch, scratch_bytes, ws)))
         return rc;
     }
-    if (dx) return conv_dgrad(lin_desc(T, l.in, l.out), SRT_BF16, SRT_IMPL_AUTO, dy, WT + l.wt_off, dx, nullptr, stream);
+    if (dx) return conv_dgrad_direct(lin_desc(T, l.in, l.out), SRT_BF16, SRT_IMPL_AUTO, dy, pw(l.w), dx, nullptr, stream);
     return SRT_OK;
   }
   srt_conv_desc pe_desc(int B) const {
@@ -162,7 +160,6 @@ struct Swin {
     return {B, I, I, 8, cfg.embed, p, p, p, 0, I / p, I / p};
   }
   int build();
-  int transposes();
   int forward(int B);
   int backward(int B, int global_batch);
   int block_fwd(Blk& k, const __nv_bfloat16* x, int B);
@@ -218,7 +215,7 @@ int Swin::build() {
 
   int rc;
   if ((rc = dalloc(&P, n_flat * 4, true)) || (rc = dalloc(&G, n_flat * 4, true)) || (rc = dalloc(&M1, n_flat * 4, true)) ||
-      (rc = dalloc(&M2, n_flat * 4, true)) || (rc = dalloc(&Pw, n_flat * 2, true)) || (rc = dalloc(&WT, n_wt * 2, true)))
+      (rc = dalloc(&M2, n_flat * 4, true)) || (rc = dalloc(&Pw, n_flat * 2, true)))
     return rc;
   const size_t B = cfg.max_batch, I = cfg.image;
   auto act = [&](__nv_bfloat16** p, size_t elems) { return dalloc(p, elems * 2, true); };
@@ -295,17 +292,6 @@ int Swin::build() {
     SRT_CHECK_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
   }
   return SRT_OK;
-}
-
-// Transposed copies of the linear weights for the data gradients (after the bf16 working copy changed).
-int Swin::transposes() {
-  int rc;
-  auto tr = [&](const Lin& l) { return filter_transpose(SRT_BF16, pw(l.w), WT + l.wt_off, l.out, 1, l.in, stream); };
-  for (Blk& k : blocks)
-    if ((rc = tr(k.qkv)) || (rc = tr(k.proj)) || (rc = tr(k.fc)) || (rc = tr(k.fc2))) return rc;
-  for (Merge& m : merges)
-    if ((rc = tr(m.red))) return rc;
-  return tr(head);
 }
 
 int Swin::block_fwd(Blk& k, const __nv_bfloat16* x, int B) {
@@ -550,7 +536,6 @@ int srt_swin_commit_params(srt_swin* h) {
   Swin* g = (Swin*)h;
   SRT_REQUIRE(g, "swin_commit_params: null handle");
   int rc = cast_f32_to_bf16(g->P, g->Pw, (int64_t)g->n_flat, g->stream);
-  if (rc == SRT_OK) rc = g->transposes();
   if (rc) return rc;
   SRT_CHECK_CUDA(cudaStreamSynchronize(g->stream));
   return SRT_OK;
@@ -591,7 +576,7 @@ int srt_swin_optimizer(srt_swin* h) {
   int rc = adamw(g->P, g->G, g->M1, g->M2, g->Pw, (int64_t)g->n_flat, g->cfg.lr, g->cfg.beta1, g->cfg.beta2, g->cfg.eps,
                  g->cfg.weight_decay, g->opt_steps, g->stream);
   if (rc) return rc;
-  return g->transposes();
+  return SRT_OK;
 }
 
 // Mean cross-entropy of the last micro-batch.
