@@ -133,8 +133,9 @@ int rmsnorm_fwd(const void* x, const float* gamma, void* y, float* mean, float* 
 int rmsnorm_bwd(const void* dy, const void* x, const float* gamma, const float* mean, const float* rstd, const void* addend,
                 void* dx, float* dgamma, int64_t rows, int C, void* scratch, size_t scratch_bytes, cudaStream_t st);
 // Rotary embedding on the heads of a [tokens][ld] matrix, in place: pairs (d, d + D/2) of every head are rotated by
-// pos * theta^(-2d/D); inverse = 1 applies the transposed rotation (the gradient).
-int rope_apply(void* x, int64_t tokens, int S, int heads, int D, int64_t ld, float theta, int inverse, cudaStream_t st);
+// pos * theta^(-2d/D); inverse = 1 applies the transposed rotation (the gradient). table: S * D floats from rope_table.
+int rope_table(float* table, int S, int D, float theta, cudaStream_t st);
+int rope_apply(void* x, const float* table, int64_t tokens, int S, int heads, int D, int64_t ld, int inverse, cudaStream_t st);
 // SwiGLU: y = silu(gate) * up for gu = [tokens][2F] (gate first); backward writes d(gu).
 int swiglu_fwd(const void* gu, void* y, int64_t tokens, int F, cudaStream_t st);
 int swiglu_bwd(const void* dy, const void* gu, void* dgu, int64_t tokens, int F, cudaStream_t st);

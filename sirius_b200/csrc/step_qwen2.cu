@@ -39,6 +39,7 @@ struct Qwen2 {
   size_t n_flat = 0;
   float *P = nullptr, *G = nullptr, *M1 = nullptr, *M2 = nullptr;
   __nv_bfloat16* Pw = nullptr;
+  float* rope = nullptr;  // cos and sin of every rotary angle
   int opt_steps = 0;
 
   struct Lin { size_t w_off; long long b_off; int in, out; };  // offsets into the flat buffers; b_off < 0 = no bias
@@ -262,6 +263,7 @@ int Qwen2::build() {
       (rc = dalloc(&M2, n_flat * 4, true)) || (rc = dalloc(&Pw, n_flat * 2, true)))
     return rc;
   if ((rc = dalloc(&ACC, n_flat * 4, true)) || (rc = dalloc(&loss_acc, 256, true))) return rc;
+  if ((rc = dalloc(&rope, (size_t)S * D * 4))) return rc;
   const size_t T = (size_t)cfg.max_batch * S;
   size_t sb = layernorm_bwd_scratch_bytes(C);
   if (colsum_scratch_bytes(QKV) > sb) sb = colsum_scratch_bytes(QKV);
@@ -289,6 +291,7 @@ int Qwen2::build() {
     SRT_CHECK_CUDA(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
     SRT_CHECK_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
   }
+  if ((rc = rope_table(rope, S, D, cfg.rope_theta, stream))) return rc;
   return alloc_activations(cfg.max_batch);
 }
 
@@ -383,7 +386,6 @@ int Qwen2::attention_backward(Layer& y, int B, float scale) {
 int Qwen2::forward(int B) {
   const int64_t T = (int64_t)B * S;
   const float scale = 1.f / sqrtf((float)D);
-  const int KO = Hq * D;  // column offset of K inside the fused projection
   int rc;
   if ((rc = join_side())) return rc;
   if ((rc = embedding_fwd(ids, pf(emb), nullptr, x0, T, S, C, stream))) return rc;
@@ -392,8 +394,7 @@ int Qwen2::forward(int B) {
     if ((rc = checkpoint())) return rc;
     if ((rc = rmsnorm_fwd(x, pf(y.n1), y.n1o, y.z1, y.r1, T, C, cfg.rms_eps, stream))) return rc;
     if ((rc = linear_fwd(y.qkv, y.n1o, y.qkv_o, nullptr, T))) return rc;
-    if ((rc = rope_apply(y.qkv_o, T, S, Hq, D, QKV, cfg.rope_theta, 0, stream))) return rc;
-    if ((rc = rope_apply(y.qkv_o + KO, T, S, Hkv, D, QKV, cfg.rope_theta, 0, stream))) return rc;
+    if ((rc = rope_apply(y.qkv_o, rope, T, S, Hq + Hkv, D, QKV, 0, stream))) return rc;  // the K heads follow the Q heads
     if ((rc = attention_forward(y, B, scale))) return rc;
     if ((rc = linear_fwd(y.o, y.att, y.x2, x, T))) return rc;
     if ((rc = rmsnorm_fwd(y.x2, pf(y.n2), y.n2o, y.z2, y.r2, T, C, cfg.rms_eps, stream))) return rc;
@@ -409,7 +410,6 @@ int Qwen2::forward(int B) {
 int Qwen2::backward(int B, int global_batch) {
   const int64_t T = (int64_t)B * S;
   const float scale = 1.f / sqrtf((float)D);
-  const int KO = Hq * D;
   int rc;
   buckets.begin_backward();
   const float gscale = 1.f / ((float)global_batch * (float)(S - 1));
@@ -444,8 +444,7 @@ int Qwen2::backward(int B, int global_batch) {
     if ((rc = linear_bwd(y.o, dx_other, y.att, datt, T))) return rc;
     if ((rc = attention_backward(y, B, scale))) return rc;
     // through the rotation (transposed), the fused projection and the first norm
-    if ((rc = rope_apply(dqkv, T, S, Hq, D, QKV, cfg.rope_theta, 1, stream))) return rc;
-    if ((rc = rope_apply(dqkv + KO, T, S, Hkv, D, QKV, cfg.rope_theta, 1, stream))) return rc;
+    if ((rc = rope_apply(dqkv, rope, T, S, Hq + Hkv, D, QKV, 1, stream))) return rc;
     if ((rc = linear_bwd(y.qkv, dqkv, y.n1o, dln, T))) return rc;
     if ((rc = join_side())) return rc;  // the next kernel overwrites dx, which this layer's first weight gradient read
     if ((rc = rmsnorm_bwd(dln, xin, pf(y.n1), y.z1, y.r1, dx_other, dx, gf(y.n1), T, C, scratch, scratch_bytes, stream)))
