@@ -1844,7 +1844,12 @@ static int conv_gather_gemm_tc_persistent(const GatherGeom& g, const void* src, 
   if (g_force_pair == 1) pair = g.Nout > 64 && g_force_bn != 64;
   if (sm_count() < 2) pair = false;
   int bn;
-  if (pair) bn = g_force_bn ? g_force_bn : (g.Nout > 128 ? 256 : 128);
+  // Width of a pair's tile: 128 columns while one wave of pairs covers the output with them. Few pairs of 256 columns are
+  // bound by their own tensor cores (512 clocks a k-block, 617 measured on 24 SMs) with the rest of the device idle; half as
+  // wide, a k-block is 24 KB per SM to load instead of 32 KB. Several waves are bound by the operand stream out of L2,
+  // which the wider tile shortens.
+  const bool one_wave = ceil_div(ceil_div(g.M, BM), 2) * ceil_div(g.Nout, 128) <= sm_count() / 2;
+  if (pair) bn = g_force_bn ? g_force_bn : (g.Nout > 128 && !one_wave ? 256 : 128);
   else bn = pick_bn(g.M, g.Nout, g_force_bn);
   p.m_tiles = ceil_div(g.M, BM);
   p.n_tiles = ceil_div(g.Nout, bn);
