@@ -383,26 +383,61 @@ int conv_large(const GatherGeom& g, const void* src, const void* Bm, void* D, co
 
 }  // namespace
 
+// Partial sums out of L2, added in split order with eight splits in flight. VEC: four elements a thread, where that still
+// leaves every SM a block; otherwise (small filters, odd counts) an element a thread.
+template <bool VEC>
 __global__ void split_reduce_kernel(const float* __restrict__ partial, float* __restrict__ out,
                                     long long n, int splits) {
   pdl_enter();
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long stride = (long long)gridDim.x * blockDim.x;
-  for (; i < n; i += stride) {
-    float s = 0.f;
-    for (int k = 0; k < splits; ++k) s += partial[(size_t)k * n + i];
-    out[i] = s;
+  if constexpr (VEC) {
+    const float4* p4 = reinterpret_cast<const float4*>(partial);
+    const long long n4 = n / 4;
+    for (; i < n4; i += stride) {
+      float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+      int k = 0;
+      for (; k + 8 <= splits; k += 8) {
+        float4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = p4[(k + u) * n4 + i];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) { s.x += v[u].x; s.y += v[u].y; s.z += v[u].z; s.w += v[u].w; }
+      }
+#pragma unroll 4
+      for (; k < splits; ++k) {
+        const float4 v = p4[k * n4 + i];
+        s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+      }
+      reinterpret_cast<float4*>(out)[i] = s;
+    }
+  } else {
+    for (; i < n; i += stride) {
+      float s = 0.f;
+      int k = 0;
+      for (; k + 8 <= splits; k += 8) {
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = partial[(size_t)(k + u) * n + i];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s += v[u];
+      }
+      for (; k < splits; ++k) s += partial[(size_t)k * n + i];
+      out[i] = s;
+    }
   }
 }
 
 int launch_split_reduce(const float* partial, float* out, long long n, int splits,
                         cudaStream_t st) {
   const int threads = 256;
-  long long blocks = (n + threads - 1) / threads;
+  const bool vec = n % 4 == 0 && (((uintptr_t)partial | (uintptr_t)out) & 15) == 0 && n / 4 >= (long long)threads * sm_count();
+  long long blocks = ((vec ? n / 4 : n) + threads - 1) / threads;
   const long long cap = (long long)sm_count() * 8;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
-  launch_pdl(split_reduce_kernel, dim3((unsigned)blocks), dim3(threads), 0, st, partial, out, n, splits);
+  launch_pdl(vec ? split_reduce_kernel<true> : split_reduce_kernel<false>, dim3((unsigned)blocks), dim3(threads), 0, st, partial, out,
+             n, splits);
   SRT_LAUNCH_CHECK();
   return SRT_OK;
 }
