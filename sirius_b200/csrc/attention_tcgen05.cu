@@ -22,8 +22,9 @@
 // the backward kernels, about 9 instructions per element at 128 lanes a clock, against 256 to 512 clocks for the
 // products of a tile; memory traffic is Q, K, V, O and their gradients once, the repeats come out of L2.
 // The score-matrix path moved 10 to 14 S x S matrices per layer through HBM.
-// Measured, 8 sequences of 1024, 12 heads: forward 81 us, backward 199 us, where the score-matrix path took 740 us for
-// both (GEMMs 276, softmax 166, transposes 298); 4 x 2048 with 14 query and 2 KV heads: 157 and 377 us against 1650 us.
+// Measured, 8 sequences of 1024, 12 heads: forward 65 us, backward 179 us, where the score-matrix path took 740 us for
+// both (GEMMs 276, softmax 166, transposes 298); 4 x 2048 with 14 query and 2 KV heads: 122 and 331 us against 1650 us.
+// (Longest rows first within a head only, instead of over the whole grid: 81, 199, 157 and 377 us.)
 // Two compute warps per scheduler (a thread with all 128 columns of a row) took 140 and 249 us: the chain of a tile
 // (product, wait, load, arithmetic, store) then leaves schedulers idle.
 //
@@ -177,8 +178,9 @@ attention_fwd_kernel(const AttFwdParams p, const __grid_constant__ CUtensorMap t
   uint32_t* tmem_ptr = (uint32_t*)(bars + 5 + 2 * FWD_NS);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nq = (p.S + TR - 1) / TR;
-  const int qi = CAUSAL ? nq - 1 - (int)blockIdx.x : (int)blockIdx.x;  // longest rows first
-  const int h = blockIdx.y, b = blockIdx.z;
+  // blocks of all heads before the next block of any: the longest rows of the whole grid go first
+  const int qi = CAUSAL ? nq - 1 - (int)blockIdx.z : (int)blockIdx.z;
+  const int h = blockIdx.x, b = blockIdx.y;
   const int n = CAUSAL ? qi + 1 : nq;  // key blocks
 
   if (tid == 0) {
@@ -431,8 +433,8 @@ attention_bwd_kernel(const AttBwdParams p, const __grid_constant__ CUtensorMap t
   uint32_t* tmem_ptr = (uint32_t*)(bars + 5 + 2 * BWD_NS);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nb = (p.S + TR - 1) / TR;
-  const int own = KV ? (int)blockIdx.x : nb - 1 - (int)blockIdx.x;  // longest loops first
-  const int h = blockIdx.y, b = blockIdx.z, hk = h / p.kv_div;
+  const int own = KV ? (int)blockIdx.z : nb - 1 - (int)blockIdx.z;  // longest loops of the whole grid first
+  const int h = blockIdx.x, b = blockIdx.y, hk = h / p.kv_div;
   const int n = KV ? nb - own : own + 1;
   constexpr int rounds = KV ? 1 : 2;
   const int first = KV ? own : 0;
@@ -638,7 +640,7 @@ attention_bwd_kernel(const AttBwdParams p, const __grid_constant__ CUtensorMap t
 }
 
 int check(const AttentionShape& a) {
-  SRT_REQUIRE(a.D == HD && a.S > 0 && a.S % 8 == 0 && a.H > 0 && a.Hkv > 0 && a.H % a.Hkv == 0 && a.B > 0 && a.B <= 65535 && a.H <= 65535,
+  SRT_REQUIRE(a.D == HD && a.S > 0 && a.S % 8 == 0 && a.H > 0 && a.Hkv > 0 && a.H % a.Hkv == 0 && a.B > 0 && a.B <= 65535 && a.S <= 65535 * TR,
               "attention: 64-channel heads, a length that is a multiple of 8 and whole head groups are required");
   return SRT_OK;
 }
@@ -668,7 +670,7 @@ int attention_fwd(const AttentionShape& a, const void* Q, const void* K, const v
   AttFwdParams p = {(bf16*)O, rows, rows ? rows + (size_t)a.B * a.H * s_pad : nullptr, a.S, s_pad, a.H, a.H / a.Hkv, ld_o, HD,
                     (long long)a.S * ld_o, scale, tc_status_device_ptr()};
   SRT_REQUIRE(p.status != nullptr, "tcgen05 status word unavailable");
-  const dim3 grid(ceil_div(a.S, TR), a.H, a.B);
+  const dim3 grid(a.H, a.B, ceil_div(a.S, TR));
   const size_t smem = fwd_smem_bytes();
   if (causal) {
     if ((rc = reserve_smem(attention_fwd_kernel<true>, smem))) return rc;
@@ -698,7 +700,7 @@ int attention_bwd_causal(const AttentionShape& a, const void* Q, const void* K, 
   AttBwdParams p = {(bf16*)dQ, nullptr, rows, rows + vec, rows + 2 * vec, a.S, s_pad, a.H, a.H / a.Hkv,
                     ld_dq, HD, (long long)a.S * ld_dq, scale, tc_status_device_ptr()};
   SRT_REQUIRE(p.status != nullptr, "tcgen05 status word unavailable");
-  const dim3 grid(ceil_div(a.S, TR), a.H, a.B);
+  const dim3 grid(a.H, a.B, ceil_div(a.S, TR));
   if ((rc = reserve_smem(attention_bwd_kernel<false>, bwd_smem_bytes(false)))) return rc;
   launch_pdl_if(early(), attention_bwd_kernel<false>, grid, dim3(BWD_THREADS), bwd_smem_bytes(false), st, p, tq, tdo, tk, tv);
   SRT_LAUNCH_CHECK();
