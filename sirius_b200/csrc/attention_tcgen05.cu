@@ -22,9 +22,10 @@
 // the backward kernels, about 9 instructions per element at 128 lanes a clock, against 256 to 512 clocks for the
 // products of a tile; memory traffic is Q, K, V, O and their gradients once, the repeats come out of L2.
 // The score-matrix path moved 10 to 14 S x S matrices per layer through HBM.
-// Measured, 8 sequences of 1024, 12 heads: forward 65 us, backward 179 us, where the score-matrix path took 740 us for
-// both (GEMMs 276, softmax 166, transposes 298); 4 x 2048 with 14 query and 2 KV heads: 122 and 331 us against 1650 us.
-// (Longest rows first within a head only, instead of over the whole grid: 81, 199, 157 and 377 us.)
+// Measured, 8 sequences of 1024, 12 heads: forward 61 us, backward 153 us, where the score-matrix path took 740 us for
+// both (GEMMs 276, softmax 166, transposes 298); 4 x 2048 with 14 query and 2 KV heads: 109 and 271 us against 1650 us.
+// (Longest rows first within a head only, instead of over the whole grid: 81, 199, 157 and 377 us; masks in every tile
+// instead of the tiles on the edge: 65, 179, 122 and 331 us.)
 // Two compute warps per scheduler (a thread with all 128 columns of a row) took 140 and 249 us: the chain of a tile
 // (product, wait, load, arithmetic, store) then leaves schedulers idle.
 //
@@ -95,6 +96,18 @@ __device__ __forceinline__ uint64_t exp2x(uint32_t s0, uint32_t s1, uint64_t sca
   asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(a));
   asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(b));
   return pair(a, b);
+}
+// Scores of columns beyond `last` (before `first`) become -inf, whose exponential is exactly zero. Only the blocks on the edge
+// call these: masks inside the loops over the columns cost every block a compare and a select per element.
+__device__ __forceinline__ void hide(uint32_t (&s)[32], int last) {
+#pragma unroll
+  for (int c = 0; c < 32; ++c)
+    if (c > last) s[c] = 0xff800000u;
+}
+__device__ __forceinline__ void hide_before(uint32_t (&s)[32], int first) {
+#pragma unroll
+  for (int c = 0; c < 32; ++c)
+    if (c < first) s[c] = 0xff800000u;
 }
 // The bounded wait of the compute warps, one outcome for the whole warp. They poll without sleeping: nothing else runs on
 // their schedulers meanwhile but each other, and a sleep would add to the serial chain of a tile.
@@ -223,9 +236,8 @@ attention_fwd_kernel(const AttFwdParams p, const __grid_constant__ CUtensorMap t
       tc_fence_before_sync();
       warp_arrive(s_free, lane);
       if (t == n - 1) {
-#pragma unroll
-        for (int c = 0; c < 64; ++c)
-          if (c > last) s[c >> 5][c & 31] = 0xff800000u;
+        hide(s[0], last);
+        hide(s[1], last - 32);
       }
       float m4[4] = {mx, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
@@ -255,6 +267,7 @@ attention_fwd_kernel(const AttFwdParams p, const __grid_constant__ CUtensorMap t
           tc_fence_before_sync();
           warp_arrive(s_free, lane);
         }
+        if (edge) hide(s, last - hf * 32);
 #pragma unroll
         for (int e = 0; e < 8; e += 2) {  // the chains of eight sums advance side by side
 #pragma unroll
@@ -262,10 +275,6 @@ attention_fwd_kernel(const AttFwdParams p, const __grid_constant__ CUtensorMap t
             const int c = i * 8 + e;
             float e0, e1;
             split(exp2x(s[c], s[c + 1], scale2, neg_max), e0, e1);
-            if (edge) {
-              if (hf * 32 + c > last) e0 = 0.f;
-              if (hf * 32 + c + 1 > last) e1 = 0.f;
-            }
             even[hf * 4 + i] += e0;
             even[hf * 4 + i] += e1;
           }
@@ -310,15 +319,9 @@ attention_fwd_kernel(const AttFwdParams p, const __grid_constant__ CUtensorMap t
           tc_fence_before_sync();
           warp_arrive(s_free, lane);
         }
+        if (edge) hide(s, last - hf * 32);
 #pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-          uint32_t v = round2(mul2(exp2x(s[c], s[c + 1], scale2, neg_max), inv2));
-          if (edge) {
-            if (hf * 32 + c > last) v &= 0xffff0000u;
-            if (hf * 32 + c + 1 > last) v &= 0x0000ffffu;
-          }
-          w[hf * 16 + c / 2] = v;
-        }
+        for (int c = 0; c < 32; c += 2) w[hf * 16 + c / 2] = round2(mul2(exp2x(s[c], s[c + 1], scale2, neg_max), inv2));
       }
       if (j > 0) {  // the previous block's P V product has read the probabilities
         ok = wait_all(o_done, (uint32_t)(j - 1) & 1u, p.status, W_ATT_COMPUTE);
@@ -487,17 +490,13 @@ attention_bwd_kernel(const AttBwdParams p, const __grid_constant__ CUtensorMap t
         tmem_ld_wait();
         tc_fence_before_sync();
         warp_arrive(s_free, lane);
-        const bool diag = t == n - 1;
+        if (t == n - 1) hide(s, row - grp * 32);  // the block on the diagonal
 #pragma unroll
         for (int e = 0; e < 8; e += 2) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const int c = i * 8 + e, col = grp * 32 + c;
-            uint32_t w = round2(mul2(exp2x(s[c], s[c + 1], scale2, neg_max), inv2));
-            if (diag) {
-              if (col > row) w &= 0xffff0000u;
-              if (col + 1 > row) w &= 0x0000ffffu;
-            }
+            const int c = i * 8 + e;
+            const uint32_t w = round2(mul2(exp2x(s[c], s[c + 1], scale2, neg_max), inv2));
             const uint32_t d = round2(pair(dp[c], dp[c + 1]));
             even[i] = fmaf(__uint_as_float(w << 16), __uint_as_float(d << 16), even[i]);
             even[i] = fmaf(__uint_as_float(w & 0xffff0000u), __uint_as_float(d & 0xffff0000u), even[i]);
@@ -536,21 +535,19 @@ attention_bwd_kernel(const AttBwdParams p, const __grid_constant__ CUtensorMap t
       tmem_ld_wait();
       tc_fence_before_sync();
       warp_arrive(s_free, lane);
-      const bool diag = KV ? it == 0 : it == n - 1;  // the block on the diagonal
+      if (KV ? it == 0 : it == n - 1) {  // the block on the diagonal: a query sees the keys up to its own position
+        if (KV) hide_before(s, row - grp * 32);
+        else hide(s, row - grp * 32);
+      }
       uint32_t wp[16], wd[16];
 #pragma unroll
       for (int c = 0; c < 32; c += 2) {
-        const int col = grp * 32 + c;
         if (KV) {
           neg_max = *reinterpret_cast<const uint64_t*>(vec + c);
           inv2 = *reinterpret_cast<const uint64_t*>(vec + 128 + c);
           neg_dot = *reinterpret_cast<const uint64_t*>(vec + 256 + c);
         }
-        uint32_t w = round2(mul2(exp2x(s[c], s[c + 1], scale2, neg_max), inv2));
-        if (diag) {
-          if (KV ? col < row : col > row) w &= 0xffff0000u;
-          if (KV ? col + 1 < row : col + 1 > row) w &= 0x0000ffffu;
-        }
+        const uint32_t w = round2(mul2(exp2x(s[c], s[c + 1], scale2, neg_max), inv2));
         wp[c >> 1] = w;
         wd[c >> 1] = round2(mul2(widen2(w), add2(widen2(round2(pair(dp[c], dp[c + 1]))), neg_dot)));
       }
@@ -661,6 +658,7 @@ int attention_s_pad(int S) { return (S + TR - 1) / TR * TR; }
 int attention_fwd(const AttentionShape& a, const void* Q, const void* K, const void* V, long long ld_qkv, void* O, long long ld_o,
                   float* rows, float scale, int causal, cudaStream_t st) {
   int rc = check(a);
+  if (!rc && !(scale > 0.f)) { set_error("attention: the score scale must be positive"); rc = SRT_ERR_INVALID; }
   if (rc) return rc;
   CUtensorMap tq, tk, tv;
   if ((rc = tmap(&tq, Q, a, a.H, ld_qkv)) || (rc = tmap(&tk, K, a, a.Hkv, ld_qkv)) || (rc = tmap(&tv, V, a, a.Hkv, ld_qkv)))
@@ -687,6 +685,7 @@ int attention_bwd_causal(const AttentionShape& a, const void* Q, const void* K, 
                          long long ld_o, float* rows, void* dQ, long long ld_dq, void* dK, void* dV, long long ld_dkv,
                          long long dkv_s1, long long dkv_s2, float scale, cudaStream_t st) {
   int rc = check(a);
+  if (!rc && !(scale > 0.f)) { set_error("attention: the score scale must be positive"); rc = SRT_ERR_INVALID; }
   if (rc) return rc;
   CUtensorMap tq, tk, tv, tdo;
   if ((rc = tmap(&tq, Q, a, a.H, ld_qkv)) || (rc = tmap(&tk, K, a, a.Hkv, ld_qkv)) || (rc = tmap(&tv, V, a, a.Hkv, ld_qkv)) ||
