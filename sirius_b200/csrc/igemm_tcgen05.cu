@@ -1105,7 +1105,8 @@ igemm_fwd_persistent(const PersistParams p, const __grid_constant__ CUtensorMap 
 // one SM is bound by the serial chain of its k-blocks (a few hundred clocks each) and leaves most of the device idle: a
 // 196 x 256 layer with 36 k-blocks has 8 tiles. The convolutions of one ResNet-152 image: 1.71 ms of device time on the
 // persistent kernel (19.4 us for the long ones), 1.32 ms with the split, which is 8 us each, mostly launch, set-up and
-// the two cluster barriers; a sentence of 128 tokens through a 3072 x 768 layer: 26.3 us before, 11 us now.
+// the two cluster barriers; a sentence of 128 tokens through a 3072 x 768 layer: 26.3 us before, 11 us now. The loads of
+// scale, shift and addend behind the barrier instead of before it made a whole image 1.26 ms instead of 1.01.
 // No load is multicast; what crosses the cluster are the accumulators.
 constexpr int SPLIT_NS = 6;
 constexpr int SPLIT_STAGE_BYTES = A_STAGE_BYTES + 64 * BK * 2;
@@ -1150,10 +1151,27 @@ igemm_infer_split(const SplitParams p, const __grid_constant__ CUtensorMap tmap_
   const uint32_t acc = *tmem_ptr;
   pdl_enter();
 
+  // What the epilogue of this thread's row reads besides the sums: its first eight columns are fetched now, beside the
+  // operand loads, and not after the cluster's barrier.
+  const int quads = 16 / S, m = m0 + tid;
+  const bool finishes = tid < BM && m < g.M;
+  float sc[8], sh[8];
+  Vec16<bf16> add;
+  auto fetch = [&](int col) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      sc[e] = p.scale ? p.scale[col + e] : 1.f;
+      sh[e] = p.shift ? p.shift[col + e] : 0.f;
+    }
+    add.raw = make_uint4(0, 0, 0, 0);
+    if (p.addend) add.load(p.addend + (size_t)m * g.Nout + col);
+  };
+  if (finishes && n0 + rank * quads * 4 < g.Nout) fetch(n0 + rank * quads * 4);
+
   if (warp < 4) {
     mbar_wait(smem_u32(acc_full), 0u, p.status, W_EPI_TMEM);
     tc_fence_after_sync();
-    const int row = warp * 32 + lane, quads = 16 / S;
+    const int row = warp * 32 + lane;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       uint32_t v[32];
@@ -1213,12 +1231,12 @@ igemm_infer_split(const SplitParams p, const __grid_constant__ CUtensorMap tmap_
   }
   __syncwarp();
   cluster_sync_all();  // the partial sums of every rank are here (release on arrival, acquire on the wait)
-  if (tid < BM && m0 + tid < g.M) {
-    const int quads = 16 / S, m = m0 + tid;
+  if (finishes) {
     for (int q = 0; q < quads; q += 2) {  // eight columns at a time (S is at most 8, so quads is even)
       const int col = n0 + (rank * quads + q) * 4;
       if (col >= g.Nout) break;  // Nout is a multiple of eight
-      float f[8];
+      if (q) fetch(col);
+      float f[8], af[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) f[e] = 0.f;
       for (int r = 0; r < S; ++r)
@@ -1227,18 +1245,9 @@ igemm_infer_split(const SplitParams p, const __grid_constant__ CUtensorMap tmap_
           const float4 v = *reinterpret_cast<const float4*>(sums + ((r * quads + q + e) * BM + tid) * 4);
           f[e * 4] += v.x; f[e * 4 + 1] += v.y; f[e * 4 + 2] += v.z; f[e * 4 + 3] += v.w;
         }
-      float af[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      if (p.addend) {
-        Vec16<bf16> a;
-        a.load(p.addend + (size_t)m * g.Nout + col);
-        a.unpack(af);
-      }
+      add.unpack(af);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        if (p.scale) f[e] *= p.scale[col + e];
-        if (p.shift) f[e] += p.shift[col + e];
-        f[e] = infer_act(f[e] + af[e], p.act);
-      }
+      for (int e = 0; e < 8; ++e) f[e] = infer_act(fmaf(f[e], sc[e], sh[e]) + af[e], p.act);
       Vec16<bf16> o;
       o.pack(f);
       o.store(p.D + (size_t)m * g.Nout + col);
