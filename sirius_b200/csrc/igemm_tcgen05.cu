@@ -1,6 +1,6 @@
 // bf16 implicit-GEMM convolution on the sm_100a tensor cores.
 //
-// Two warp-specialised kernels:
+// Warp-specialised kernels:
 //
 //   igemm_fwd_persistent<BN, NS, PAIR, INFER>   fprop and dgrad.  D[m][n] = sum_k A(m,k) B[n][k]
 //       Persistent: one CTA (or one CTA pair, cta_group::2) per SM walks output tiles of 128 (256 for a pair)
@@ -17,6 +17,8 @@
 //       on its own mbarrier per (group, accumulator buffer) so that a waiter never falls two phases behind.
 //       The epilogue converts to bf16, adds bias / residual, optionally accumulates per-channel sums for
 //       BatchNorm, stages the slab in shared memory and stores it with TMA.
+//   igemm_infer_split                    fprop in inference with few tiles: a cluster shares a tile's reduction and adds its
+//       accumulators through shared memory (INFER instances of the persistent kernel otherwise).
 //   igemm_wgrad_kernel                   filter gradient.  dW[k][j] = sum_pix dy[pix][k] X(pix,j)
 //       192 threads, one 128-filter tile per CTA.
 //       A: dy block, 64 pixels x 128 filters per stage by TMA (MN-major, two 64-wide boxes).

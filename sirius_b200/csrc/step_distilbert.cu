@@ -7,7 +7,8 @@
 // Same building blocks as the training executors: activations are [tokens][features] bf16 rows, linear layers
 // run on the tcgen05 implicit-GEMM kernels (bias and residual add in the epilogue), Q, K and V come from one
 // fused [tokens][3*dim] projection (the three weight matrices sit back to back in the flat parameter buffer) and
-// the attention products are batched tcgen05 GEMMs addressing the heads in place. Activations come from the
+// 64-channel heads take the fused attention kernel, other sizes batched tcgen05 GEMMs that address the heads in place.
+// Activations come from the
 // INFERENCE allocator of a page pool when one is attached, so that a request that finds no memory triggers the
 // handover from the colocated trainer, and go back to the pool when the worker idles.
 #include <string.h>

@@ -4,7 +4,8 @@
 // projection tied to the token table, next-token cross-entropy, AdamW.
 //
 // Same layout as the GPT-2 executor: [tokens][features] bf16 rows, linear layers on the tcgen05 implicit-GEMM
-// kernels, attention over 4-D tensor maps (one kernel for 64-channel heads, batched GEMMs for other sizes). Q, K and V live in one fused
+// kernels, attention over 4-D tensor maps (fused kernels for 64-channel heads, batched GEMMs for other sizes). Q, K and V
+// live in one fused
 // [tokens][(Hq + 2 Hkv) D] projection (their weights are adjacent rows of one matrix), gate and up in one
 // [tokens][2 F] projection. Several query heads read one KV head through the batch divisor of the GEMM; the
 // KV gradients are produced per query head and summed per group.
@@ -314,7 +315,8 @@ int Qwen2::alloc_activations(int B) {
   if ((rc = act(&x0, T * C))) return rc;
   for (Layer& y : layers) {
     if ((rc = act(&y.n1o, T * C)) || (rc = act(&y.qkv_o, T * QKV)) ||
-        (rc = flash ? actf(&y.rows, attention_rows_floats(B, S, Hq)) : act(&y.Pm, BH * S * S)) || (rc = act(&y.att, T * Hq * D)) || (rc = act(&y.x2, T * C)) || (rc = act(&y.n2o, T * C)) ||
+        (rc = flash ? actf(&y.rows, attention_rows_floats(B, S, Hq)) : act(&y.Pm, BH * S * S)) ||
+        (rc = act(&y.att, T * Hq * D)) || (rc = act(&y.x2, T * C)) || (rc = act(&y.n2o, T * C)) ||
         (rc = act(&y.gu_o, T * 2 * F)) || (rc = act(&y.act, T * F)) || (rc = act(&y.xout, T * C)))
       return rc;
     if ((rc = zeros(&y.z1, T)) || (rc = actf(&y.r1, T)) || (rc = zeros(&y.z2, T)) || (rc = actf(&y.r2, T))) return rc;
@@ -354,7 +356,8 @@ int Qwen2::attention_backward(Layer& y, int B, float scale) {
   const long long SS = (long long)S * S;
   int rc;
   if (attention_supported(D)) {
-    if ((rc = attention_bwd_causal({B, S, Hq, Hkv, D}, y.qkv_o, y.qkv_o + KO, y.qkv_o + VO, QKV, datt, KO, y.rows, dqkv, QKV, dkv_h, t1, D, (long long)S * D, (long long)Hq * S * D, scale, stream)))
+    if ((rc = attention_bwd_causal({B, S, Hq, Hkv, D}, y.qkv_o, y.qkv_o + KO, y.qkv_o + VO, QKV, datt, KO, y.rows,
+                                   dqkv, QKV, dkv_h, t1, D, (long long)S * D, (long long)Hq * S * D, scale, stream)))
       return rc;
     if ((rc = head_group_sum(t1, dqkv + VO, B, S, Hq, group, D, QKV, stream))) return rc;
     return head_group_sum(dkv_h, dqkv + KO, B, S, Hq, group, D, QKV, stream);
