@@ -287,8 +287,9 @@ int srt_step_reserve_activations(srt_step* s, int B);
 int srt_step_shrink_activations(srt_step* s, int B, size_t* released_bytes);
 /* Kill batch (ColocateStub on kColocateAdjustL1, pytorch/torch_col/csrc/control_stub.cc:486-510; the
  * reference drops the launches still queued in xsched): any thread may raise the flag; forward and
- * backward test it between units and return SRT_ERR_ABORTED, and never run more than 8 units ahead of
- * the GPU, so the stream drains within a bounded time. Clear the flag before the next micro-batch. */
+ * backward test it between units and return SRT_ERR_ABORTED, and a training pass never runs more than 8
+ * units ahead of the GPU, so the stream drains within a bounded time. An inference pass is queued whole: it
+ * ends within its own few milliseconds. Clear the flag before the next micro-batch. */
 int srt_step_request_abort(srt_step* s, int on);
 /* The pre-launch hook of the reference (pytorch/torch_col/csrc/init.cc:43-71) sets the TPC mask before
  * every kernel. With on != 0 the step does the equivalent between units: it reads the process-wide mask
