@@ -503,6 +503,7 @@ class _DistNamespace:
         pol = {'fix': 0, 'simple': 1, 'by_performance': 2}[policy.lower()]
         call("srt_dbd_init", _dist_h, dataset_size, input_batch_size, global_batch_size, int(lazy), pol)
         _DynamicBatchDistirbutor._lazy_distributing = bool(lazy)
+        _DynamicBatchDistirbutor._ledger = _dist_h
 
     @staticmethod
     def init_train_performance_model(): pass  # the table lives in the DistTrainSync segment already
@@ -511,6 +512,10 @@ class _DistNamespace:
 class _DynamicBatchDistirbutor:
     """Static facade over the shared ledger (cython/dist.pyx:84-146)."""
     _lazy_distributing = False
+    _ledger = None   # the segment the distributor was initialised on
+
+    @staticmethod
+    def inited() -> bool: return bool(_dist_h) and _DynamicBatchDistirbutor._ledger is _dist_h
 
     @staticmethod
     def _ranges(batch_range_vec):

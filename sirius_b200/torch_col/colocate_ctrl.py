@@ -170,7 +170,7 @@ class ColocateCtrl(CtrlBase):
             # an adjust may have arrived during the critical section: nothing is executing now
             if _C.get_train_world_size() == 1 and self._stub.cmd == CtrlEvent.kColocateAdjustL1:
                 with EventManager.record_duration_event('adjust_after_step'):
-                    self.adjust()
+                    self.adjust_outside_batch()
         else:
             self._stub.StepsNoInteruptBegin()
             try:
@@ -182,6 +182,17 @@ class ColocateCtrl(CtrlBase):
         if self.train_mode == TrainMode.COLOCATE_L1:
             return self.adjust_l1()
         return self.adjust_l2()
+
+    def adjust_outside_batch(self):
+        """An L1 adjust taken while no micro-batch is in flight (a job of one rank). What Trainer.handle_abort_batch does
+        after the reply of a killed batch is due here as well: the next adjust is again a request to release memory (until
+        then the stub answers every adjust on the spot), the announced batch size counts from the next micro-batch on
+        (a larger one would be mapped on pages that inference holds by then), and kInferExit may grow it back."""
+        self.adjust()
+        self.set_killed_batch_recover()
+        if _C._DynamicBatchDistirbutor.inited():
+            _C._DynamicBatchDistirbutor.distribute_batch(True, True, False)
+        self.set_killed_batch_reconfiged()
 
     def adjust_l1(self):
         """Release the activation set, return empty pages to the pool, reply (colocate_ctrl.py:413-445)."""

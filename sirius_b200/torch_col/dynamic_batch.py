@@ -291,7 +291,10 @@ class DynamicBatchDataset(torch.utils.data.IterableDataset):
         if self.col_ctrl.train_mode.is_colocate():
             while bs <= 0:
                 _C.update_current_batch_size(bs)
-                if self.col_ctrl._stub.cmd in (CtrlEvent.kColocateAdjustL1, CtrlEvent.kColocateAdjustL2):
+                cmd = self.col_ctrl._stub.cmd
+                if cmd == CtrlEvent.kColocateAdjustL1 and _C.get_train_world_size() == 1:
+                    self.col_ctrl.adjust_outside_batch()
+                elif cmd in (CtrlEvent.kColocateAdjustL1, CtrlEvent.kColocateAdjustL2):
                     self.col_ctrl.release_and_reply()
                 time.sleep(1e-3)
                 bs = self.get_next_batch_size()

@@ -77,7 +77,7 @@ def _trainer(scenario, comm_name, dist_name, q):
 
     def end_after_command():
         end()
-        if plan["cid"] is not None and plan["n"] == plan["at"]:   # the command is in before the trainer looks
+        if scenario != "zero" and plan["n"] == plan["at"]:         # the command is in before the trainer looks
             _until(lambda: stub.cmd == CtrlEvent.kColocateAdjustL1, "the control thread never took the adjust in")
 
     stub.StepsNoInteruptBegin, stub.StepsNoInteruptEnd = begin_with_adjust, end_after_command
