@@ -24,6 +24,7 @@ the adjust to the return of the wait for Done, per GiB of pages that became free
 from __future__ import annotations
 
 import argparse
+import contextlib
 import ctypes as C
 import json
 import os
@@ -137,8 +138,35 @@ def trainer_main(a):
 
 
 # ------------------------------------------------------------------------------------------------------ server
+def _log_tail(path, n=1500):
+    try:
+        with open(path) as f:
+            return f.read()[-n:]
+    except OSError:
+        return ""
+
+
+def _end_trainer(launcher, result):
+    """Ends the training process, whatever state the run left it in: asks first, then kills."""
+    if launcher not in _CHILDREN:
+        return                                           # seen to exit
+    with open(result + ".stop", "w") as f:
+        f.write("stop")
+    if launcher.wait(20000) is None:
+        launcher.kill()
+        launcher.wait(20000)
+    _CHILDREN.remove(launcher)
+
+
 def run(duration_s=30.0, rate=50.0, policy="per-request", idle_ms=500.0, batch=64, seed=0, sm_partition=True,
         multi_gib=False):
+    # Whatever ends the run, the trainer, the channel and the pool end with it: a pool that stayed behind would be taken
+    # for the next run's, under a name its trainer does not know.
+    with contextlib.ExitStack() as cleanup:
+        return _run(cleanup, duration_s, rate, policy, idle_ms, batch, seed, sm_partition, multi_gib)
+
+
+def _run(cleanup, duration_s, rate, policy, idle_ms, batch, seed, sm_partition, multi_gib):
     import torch
     from . import _lib
     from ._lib import call
@@ -164,39 +192,70 @@ def run(duration_s=30.0, rate=50.0, policy="per-request", idle_ms=500.0, batch=6
     probe_pool.close()
     pool_bytes = (train_pages + 1) * page
     call("srt_pool_init", 0, pool_bytes, 1)             # the shared pool; the trainer attaches to it
+    cleanup.callback(call, "srt_pool_shutdown", 0)
     pool = C.c_void_p()
     call("srt_pool_default", 0, C.byref(pool))
     stat = lambda w: _lib.lib().srt_pool_stat(pool, w)
     FREE_PAGES = 4
 
     comm = PyInfTraCommunicator(True, True, 1)          # default name: from SIRIUS_PORT
+    cleanup.callback(comm.close)
     slope_mb = train_pages * page / batch / 2 ** 20
     adj_cfg = AdjusterConfig(0.0, slope_mb, 0, 0, 1500.0, 1, 1)
     adj = C.c_void_p()
     call("srt_adjuster_create", comm._h, C.byref(adj_cfg), C.byref(adj))
+    cleanup.callback(call, "srt_adjuster_destroy", adj)
     ctl = Controller(comm, adj, ServeMode.COLOCATE_L1)
+    cleanup.callback(ctl.close)
     resmgr = ResourceManager(pool, adj)
 
     sd = _seeded_state(ARCH)
     infer = ResNetStep(arch=ARCH, max_batch=1, image=IMAGE, dtype="bf16", pool=pool, pool_kind=INFER)
+    cleanup.callback(infer.close)
     infer.load_state_dict(sd)
     infer_bytes = infer.memory_bytes()[1]
     infer_pages = stat(5) // page - stat(FREE_PAGES)
     infer.release_activations()
 
     result = os.path.join(tempfile.gettempdir(), f"srt_colocate_{port}.json")
+    log_path = os.path.join(tempfile.gettempdir(), f"srt_colocate_{port}.log")
     launcher = TrainLauncher(ServeMode.COLOCATE_L1, use_xsched=True, use_shared_tensor_train=True,
                              cuda_memory_pool_gb=pool_bytes / 2 ** 30, dynamic_sm_partition=sm_partition)
     args = f"role=trainer batch={batch} result={result} max-seconds={duration_s + 120}" + ("" if sm_partition else " no-sm-partition")
     launcher.launch(os.path.abspath(__file__), args, interpreter=sys.executable,
-                    log_path=os.path.join(tempfile.gettempdir(), f"srt_colocate_{port}.log"))
+                    log_path=log_path)
     _CHILDREN.append(launcher)
+    for f in (result, result + ".ready", result + ".stop"):
+        cleanup.callback(lambda f=f: os.path.exists(f) and os.unlink(f))
+    cleanup.callback(_end_trainer, launcher, result)
     ctl.set_train_pid(launcher.pid)
+
+    status = None                                       # exit status of the trainer
+
+    def trainer_exited(timeout_ms=0):
+        nonlocal status
+        if launcher in _CHILDREN:
+            status = launcher.wait(timeout_ms)
+            if status is not None:
+                _CHILDREN.remove(launcher)
+        return launcher not in _CHILDREN
+
+    def wait_adjust_done(cid, limit_s=30):
+        """A trainer that has exited never answers: say so, with the end of its log, instead of waiting the limit out."""
+        t1 = time.time()
+        while True:
+            try:
+                return ctl.wait_colocate_adjust_done(0, cid, 1000)
+            except _lib.SrtError as e:
+                if trainer_exited():
+                    raise RuntimeError(f"{e}; the training process has exited: {_log_tail(log_path)}") from e
+                if time.time() - t1 > limit_s:
+                    raise
+
     t0 = time.time()
     while not os.path.exists(result + ".ready"):
-        if launcher.wait(0) is not None or time.time() - t0 > 300:
-            raise RuntimeError("the training process did not come up: " + open(
-                os.path.join(tempfile.gettempdir(), f"srt_colocate_{port}.log")).read()[-2000:])
+        if trainer_exited() or time.time() - t0 > 300:
+            raise RuntimeError("the training process did not come up: " + _log_tail(log_path))
         time.sleep(0.01)
     if stat(FREE_PAGES) >= infer_pages:
         raise RuntimeError("pool sizing: inference fits beside training without a handover")
@@ -244,7 +303,7 @@ def run(duration_s=30.0, rate=50.0, policy="per-request", idle_ms=500.0, batch=6
             t1 = time.perf_counter()
             if n.value:
                 cid = ctl.colocate_infer_require_adjust(0, [max(plan[0], 1)])
-                ctl.wait_colocate_adjust_done(0, cid, 30000)
+                wait_adjust_done(cid)
             dt = (time.perf_counter() - t1) * 1e3
             freed = (stat(FREE_PAGES) - free_before) * page
             handover.append((dt, freed))
@@ -279,7 +338,7 @@ def run(duration_s=30.0, rate=50.0, policy="per-request", idle_ms=500.0, batch=6
         free_before = stat(FREE_PAGES)
         t1 = time.perf_counter()
         cid = ctl.colocate_infer_require_adjust(0, [small])
-        ctl.wait_colocate_adjust_done(0, cid, 30000)
+        wait_adjust_done(cid)
         dt = (time.perf_counter() - t1) * 1e3
         freed = (stat(FREE_PAGES) - free_before) * page
         if freed > 0:
@@ -294,15 +353,9 @@ def run(duration_s=30.0, rate=50.0, policy="per-request", idle_ms=500.0, batch=6
     ctl.inference_workload_done()
     with open(result + ".stop", "w") as f:
         f.write("stop")
-    status = launcher.wait(120000)
-    if status is None:
+    if not trainer_exited(120000):
         launcher.kill()
-    if launcher in _CHILDREN:
-        _CHILDREN.remove(launcher)
     tr = json.load(open(result)) if os.path.exists(result) else {}
-    for f in (result, result + ".ready", result + ".stop"):
-        if os.path.exists(f):
-            os.unlink(f)
     # training throughput inside the server's window, from the trainer's per-epoch marks
     inside = [(t, s) for t, s in tr.get("marks", []) if t_begin <= t <= t_stop]
     if len(inside) >= 2:
@@ -337,11 +390,6 @@ def run(duration_s=30.0, rate=50.0, policy="per-request", idle_ms=500.0, batch=6
     }
     if policy == "cold-request":
         out["idle_ms"] = idle_ms
-    infer.close()
-    ctl.close()
-    call("srt_adjuster_destroy", adj)
-    comm.close()
-    call("srt_pool_shutdown", 0)
     return out
 
 
