@@ -124,11 +124,14 @@ int conv_fprop_infer(const srt_conv_desc& d, int dtype, int impl, const void* x,
   SRT_REQUIRE(!(dtype == SRT_F32 && impl == SRT_IMPL_TCGEN05), "conv: tcgen05 path is bf16 only");
   GatherGeom g = make_fprop_geom(d);
   if (use_tc(dtype, impl)) return conv_infer_tc(g, x, w, y, ep, st);
-  SRT_REQUIRE(conv_fprop_infer_supported(d, dtype, impl) && conv_infer_simt_ok(g, x, w, y), "conv: no inference epilogue for this shape");
+  SRT_REQUIRE(conv_fprop_infer_supported(d, dtype, impl), "conv: no inference epilogue for this shape");
   return conv_infer_simt(g, x, w, y, ep, st);
 }
-// bf16 on the CUDA cores is a cross-check without an epilogue of its own; fp32 has no GELU
-bool conv_fprop_infer_supported(const srt_conv_desc& d, int dtype, int impl) { return use_tc(dtype, impl) || dtype == SRT_F32; }
+// bf16 on the CUDA cores is a cross-check without an epilogue of its own; fp32 has no GELU. A shape that the kernel behind
+// the epilogue cannot take is not supported either: callers then run the convolution and what follows it one by one.
+bool conv_fprop_infer_supported(const srt_conv_desc& d, int dtype, int impl) {
+  return use_tc(dtype, impl) || (dtype == SRT_F32 && conv_infer_simt_ok(make_fprop_geom(d)));
+}
 
 bool conv_fprop_stats_supported(const srt_conv_desc& d, int dtype, int impl) {
   return use_tc(dtype, impl) && conv_col_stats_available() && d.C % 8 == 0 && d.K % 8 == 0;

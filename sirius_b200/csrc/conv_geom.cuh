@@ -88,7 +88,7 @@ struct InferEpilogue {
 // Declared here, defined in conv_simt.cu / igemm_tcgen05.cu.
 bool conv_dgrad_direct_ok(const srt_conv_desc& d);
 int conv_dgrad_direct_tc(const GatherGeom& g, const void* dy, const void* w, void* dx, const srt_conv_epilogue* ep, cudaStream_t st);
-bool conv_infer_simt_ok(const GatherGeom& g, const void* src, const void* Bm, const void* D);
+bool conv_infer_simt_ok(const GatherGeom& g);
 int conv_infer_simt(const GatherGeom& g, const void* src, const void* Bm, void* D, const InferEpilogue& ep, cudaStream_t st);
 int conv_infer_tc(const GatherGeom& g, const void* src, const void* Bm, void* D, const InferEpilogue& ep, cudaStream_t st);
 int conv_gather_gemm_simt(const GatherGeom& g, int dtype, const void* src, const void* Bm, void* D,

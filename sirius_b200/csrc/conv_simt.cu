@@ -188,15 +188,16 @@ __device__ __forceinline__ uint64_t twice(float v) {
 template <int BN_>
 __global__ void __launch_bounds__(LNT, 2)
 gather_gemm_f32_large(const GatherGeom g, const float* __restrict__ src, const float* __restrict__ Bm, float* __restrict__ D,
-                      const LargeEpilogue ep, int splits) {
+                      const LargeEpilogue ep, int log2_splits) {
   constexpr int TN = BN_ / 16, NB = BN_ / 64;  // outputs per thread along n; B vectors a thread fetches per k-block
   constexpr int AP = LBM + 4, BP = BN_ + 4;
   extern __shared__ __align__(16) float sm[];  // two stages of A [16][AP] and B [16][BP]; then the tile of partial sums
   const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  const int m0 = (int)blockIdx.y * LBM, n0 = (int)blockIdx.z * BN_;
-  const int rank = (int)blockIdx.x;  // the cluster lies along x
-  const int nkb = (g.Kg + LBK - 1) / LBK;
-  const int kb0 = (int)((long long)nkb * rank / splits), kb1 = (int)((long long)nkb * (rank + 1) / splits);
+  // x: row tiles (2^31 - 1 blocks at most; y and z end at 65535), each as a cluster of `splits` blocks; y: column tiles
+  const int splits = 1 << log2_splits, rank = (int)blockIdx.x & (splits - 1);
+  const int m0 = ((int)blockIdx.x >> log2_splits) * LBM, n0 = (int)blockIdx.y * BN_;
+  const int nkb = (g.Kg + LBK - 1) / LBK;  // below 2^27: the products fit
+  const int kb0 = nkb * rank >> log2_splits, kb1 = nkb * (rank + 1) >> log2_splits;
   const int lrow = t >> 2, lk = (t & 3) * 4;
 
   // two rows of A per thread: the source position of filter tap (0, 0)
@@ -320,7 +321,7 @@ gather_gemm_f32_large(const GatherGeom g, const float* __restrict__ src, const f
     for (int j = 0; j < TN / 4; ++j)
       *reinterpret_cast<float4*>(sm + (i < 4 ? ty * 4 + i : 64 + ty * 4 + i - 4) * BN_ + j * 64 + tx * 4) = quad(i, j);
   ptx::cluster_sync_all();
-  const int share = LBM / splits;  // rows this CTA finishes
+  const int share = LBM >> log2_splits;  // rows this CTA finishes
   for (int q = t; q < share * (BN_ / 4); q += LNT) {
     const int row = rank * share + q / (BN_ / 4), col = (q % (BN_ / 4)) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -336,25 +337,26 @@ gather_gemm_f32_large(const GatherGeom g, const float* __restrict__ src, const f
 // Tile width and cluster size. 128 columns where the output has as many and the cluster can still fill the device; a
 // reduction is split while the grid stays within two CTAs per SM and every part keeps four k-blocks. Clusters beyond a CTA
 // pair only on the whole device: a partition of it may have no room for one.
-struct LargePlan { int bn, splits; };
+struct LargePlan { int bn, log2_splits; };
 LargePlan plan_large(const GatherGeom& g, bool may_split) {
   const int mt = ceil_div(g.M, LBM), nkb = ceil_div(g.Kg, LBK), room = 2 * sm_count();
-  const int most = !may_split ? 1 : sm_limit() == 0 ? 8 : 2;
+  const int most = !may_split ? 0 : sm_limit() == 0 ? 3 : 1;  // log2 of the largest cluster
   LargePlan p;
-  p.bn = g.Nout > 64 && (long long)mt * ceil_div(g.Nout, 128) * most >= sm_count() ? 128 : 64;
+  p.bn = g.Nout > 64 && ((long long)mt * ceil_div(g.Nout, 128) << most) >= sm_count() ? 128 : 64;
   const long long tiles = (long long)mt * ceil_div(g.Nout, p.bn);
-  p.splits = most;
-  while (p.splits > 1 && (tiles * p.splits > room || nkb < 4 * p.splits)) p.splits /= 2;
+  p.log2_splits = most;
+  while (p.log2_splits > 0 && (tiles << p.log2_splits > room || nkb < 4 << p.log2_splits)) --p.log2_splits;
   return p;
 }
 template <int BN_>
-int launch_large(const GatherGeom& g, const float* src, const float* Bm, float* D, const LargeEpilogue& ep, int splits,
+int launch_large(const GatherGeom& g, const float* src, const float* Bm, float* D, const LargeEpilogue& ep, int log2_splits,
                  cudaStream_t st) {
+  const int splits = 1 << log2_splits;
   constexpr size_t stages = 2 * LBK * (LBM + 4 + BN_ + 4) * sizeof(float), tile = LBM * BN_ * sizeof(float);
   constexpr size_t smem = stages > tile ? stages : tile;
   SRT_CHECK_CUDA(cudaFuncSetAttribute(gather_gemm_f32_large<BN_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(splits, ceil_div(g.M, LBM), ceil_div(g.Nout, BN_));
+  cfg.gridDim = dim3(ceil_div(g.M, LBM) * splits, ceil_div(g.Nout, BN_));
   cfg.blockDim = dim3(LNT);
   cfg.dynamicSmemBytes = splits > 1 ? smem : stages;
   cfg.stream = st;
@@ -365,20 +367,22 @@ int launch_large(const GatherGeom& g, const float* src, const float* Bm, float* 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = splits > 1 ? 1 : 0;
-  SRT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gather_gemm_f32_large<BN_>, g, src, Bm, D, ep, splits));
+  SRT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gather_gemm_f32_large<BN_>, g, src, Bm, D, ep, log2_splits));
   SRT_LAUNCH_CHECK();
   return SRT_OK;
 }
-// The large-tile kernel reads and writes whole 16-byte vectors.
+// The large-tile kernel reads and writes whole 16-byte vectors. Column tiles lie on grid y.
+bool large_shape_ok(const GatherGeom& g) {
+  return (!g.dgrad || g.stride == 1) && g.src_c % 4 == 0 && g.Kg % 4 == 0 && g.Nout % 4 == 0 && ceil_div(g.Nout, 64) <= 65535;
+}
 bool large_ok(const GatherGeom& g, const void* src, const void* Bm, const void* D) {
-  return (!g.dgrad || g.stride == 1) && g.src_c % 4 == 0 && g.Kg % 4 == 0 && g.Nout % 4 == 0 && ceil_div(g.M, LBM) <= 65535 &&
-         (((uintptr_t)src | (uintptr_t)Bm | (uintptr_t)D) & 15) == 0;
+  return large_shape_ok(g) && (((uintptr_t)src | (uintptr_t)Bm | (uintptr_t)D) & 15) == 0;
 }
 int conv_large(const GatherGeom& g, const void* src, const void* Bm, void* D, const LargeEpilogue& ep, bool may_split,
                cudaStream_t st) {
   const LargePlan p = plan_large(g, may_split);
-  return p.bn == 128 ? launch_large<128>(g, (const float*)src, (const float*)Bm, (float*)D, ep, p.splits, st)
-                     : launch_large<64>(g, (const float*)src, (const float*)Bm, (float*)D, ep, p.splits, st);
+  return p.bn == 128 ? launch_large<128>(g, (const float*)src, (const float*)Bm, (float*)D, ep, p.log2_splits, st)
+                     : launch_large<64>(g, (const float*)src, (const float*)Bm, (float*)D, ep, p.log2_splits, st);
 }
 
 }  // namespace
@@ -465,8 +469,9 @@ int conv_gather_gemm_simt(const GatherGeom& g, int dtype, const void* src, const
   return gather_gemm_simt_launch<__nv_bfloat16>(g, src, Bm, D, ep, st);
 }
 
-bool conv_infer_simt_ok(const GatherGeom& g, const void* src, const void* Bm, const void* D) { return large_ok(g, src, Bm, D); }
+bool conv_infer_simt_ok(const GatherGeom& g) { return large_shape_ok(g); }
 int conv_infer_simt(const GatherGeom& g, const void* src, const void* Bm, void* D, const InferEpilogue& ep, cudaStream_t st) {
+  SRT_REQUIRE(large_ok(g, src, Bm, D), "conv: unaligned tensor");
   const LargeEpilogue e = {ep.scale, ep.shift, (const float*)ep.addend, nullptr, ep.act == ACT_RELU};
   return conv_large(g, src, Bm, D, e, true, st);
 }
