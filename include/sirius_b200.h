@@ -69,9 +69,11 @@ int srt_conv_dgrad(const srt_conv_desc* d, int dtype, int impl, const void* dy, 
 int srt_conv_wgrad(const srt_conv_desc* d, int dtype, int impl, const void* dy, const void* x,
                    float* dw, void* scratch, size_t scratch_bytes, void* stream);
 size_t srt_conv_wgrad_scratch_bytes(const srt_conv_desc* d, int dtype, int impl);
-/* wt[C,R,S,K] = transpose of w[K,R,S,C] (same dtype). */
+/* The data gradient on w[K,R,S,C] itself, without a transposed copy: bf16 on the tensor cores, stride 1, K % 64 == 0 or a
+ * 1x1 filter. */
 int srt_conv_dgrad_direct(const srt_conv_desc* d, int dtype, int impl, const void* dy, const void* w, void* dx,
-                          const srt_conv_epilogue* ep, void* stream); /* w[K,R,S,C] itself; bf16, stride 1, K % 64 == 0 or 1x1 */
+                          const srt_conv_epilogue* ep, void* stream);
+/* wt[C,R,S,K] = transpose of w[K,R,S,C] (same dtype). */
 int srt_conv_filter_transpose(const srt_conv_desc* d, int dtype, const void* w, void* wt,
                               void* stream);
 

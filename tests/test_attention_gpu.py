@@ -47,7 +47,7 @@ def by_score_matrix(qkv, do, B, S, H, scale):
     return out, dqkv
 
 
-# one key, a tile's edges and remainders, several tiles with a ragged last one; grouped and plain heads
+# eight positions (the shortest length there is), a tile's edges and remainders, several tiles with a ragged last one; grouped and plain heads
 @pytest.mark.parametrize("B,S,H,Hkv,gain", [(1, 8, 1, 1, 1.0), (2, 72, 3, 3, 1.0), (1, 128, 2, 1, 1.0), (2, 136, 4, 2, 1.0),
                                             (1, 328, 7, 1, 1.0), (2, 640, 2, 2, 4.0), (1, 1024, 3, 3, 1.0)])
 @pytest.mark.parametrize("causal", [1, 0])
