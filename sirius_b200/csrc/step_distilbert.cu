@@ -284,6 +284,15 @@ int srt_bert_forward(srt_bert* h, int B) {
   return g->forward(B);
 }
 
+// bf16 to fp32. Through restricted pointers the compiler makes it a vector loop. Element by element (the source pointer read
+// again for each, for all it knows) its speed depended on where the linker had put the loop: a result of 1.5 M values took
+// 1.11 ms or 1.47 ms in whole, 1.12 ms with this.
+static void widen(const uint16_t* __restrict__ from, float* __restrict__ to, size_t n) {
+  for (size_t i = 0; i < n; ++i) {
+    const uint32_t bits = (uint32_t)from[i] << 16;
+    memcpy(&to[i], &bits, 4);
+  }
+}
 int srt_bert_output(srt_bert* h, float* host, int B) {
   Bert* g = (Bert*)h;
   SRT_REQUIRE(g && host && B > 0 && B <= g->cfg.max_batch && g->out, "bert_output: run a forward pass first");
@@ -298,11 +307,8 @@ int srt_bert_output(srt_bert* h, float* host, int B) {
   }
   for (int k = 0; k < parts; ++k) {
     SRT_CHECK_CUDA(cudaEventSynchronize(g->stage_ev[k]));
-    const size_t end = std::min(n, (size_t)(k + 1) * part);
-    for (size_t i = (size_t)k * part; i < end; ++i) {
-      const uint32_t bits = (uint32_t)g->stage[i] << 16;
-      memcpy(&host[i], &bits, 4);
-    }
+    const size_t begin = (size_t)k * part;
+    widen(g->stage + begin, host + begin, std::min(n, begin + part) - begin);
   }
   return SRT_OK;
 }
