@@ -14,6 +14,9 @@ pytestmark = pytest.mark.gpu
 
 def test_a_run_after_a_failed_run(monkeypatch):
     pytest.importorskip("torchvision")
+    for name in [n for n in os.environ if n.startswith(("COLTRAIN_", "SIRIUS_B200_COMM", "SIRIUS_B200_DIST"))]:
+        monkeypatch.delenv(name)                       # what other tests left for trainers of their own
+    monkeypatch.setenv("SIRIUS_PORT", "0")             # set by the run; the old value comes back afterwards
     pids = []
     real_pid, real_wait = Controller.set_train_pid, Controller.wait_colocate_adjust_done
     monkeypatch.setattr(Controller, "set_train_pid", lambda self, pid: (pids.append(pid), real_pid(self, pid)))
