@@ -43,9 +43,9 @@ METRIC, UNIT = "train samples/s", "samples/s"
 # one training step, divided by the family's launches): the one-pass ncu capture of a whole step summarised in
 # profiles/resnet152_bf16_b64_step_launch_list.md. A benchmark run cannot be profiled while it is timed, so these are
 # constants of that capture; they change when the kernels do.
-DRAM_BYTES_PER_LAUNCH = {"batchnorm": 23500512, "conv_fprop_dgrad": 24757257, "conv_wgrad": 27412543,
-                         "optimizer": 8842468, "other": 32372448}
-KERNEL_LAUNCHES_PER_STEP = {"batchnorm": 609, "conv_fprop_dgrad": 310, "conv_wgrad": 266, "optimizer": 157, "other": 8}
+DRAM_BYTES_PER_LAUNCH = {"batchnorm": 23393597, "conv_fprop_dgrad": 24641883, "conv_wgrad": 27058994,
+                         "optimizer": 159895776, "other": 32336096}
+KERNEL_LAUNCHES_PER_STEP = {"batchnorm": 657, "conv_fprop_dgrad": 338, "conv_wgrad": 311, "optimizer": 8, "other": 8}
 REGIONS = 3               # timed regions per number; the median is reported
 WORKLOAD = "ResNet-152 train step (fwd+bwd+SGD-momentum), bf16, batch 64 per GPU, 3x224x224 N(0,1)"
 

@@ -1589,6 +1589,7 @@ int launch_wgrad_pair(const WgradParams& p, const CUtensorMap& tdy, const CUtens
   cfg.attrs = attr;
   cfg.numAttrs = 2;
   SRT_CHECK_CUDA(cudaLaunchKernelEx(&cfg, igemm_wgrad_pair, p, tdy, tx, tout));
+  SRT_LAUNCH_CHECK();
   return SRT_OK;
 }
 
