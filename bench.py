@@ -368,7 +368,7 @@ def run_ours(args):
                     # stated do not depend on it
                     col[key] = colocate_proc.run(duration_s=secs, policy=policy, multi_gib=(key == "cold_request"))
                 except Exception as e:  # noqa: BLE001
-                    col[key] = {"error": f"{type(e).__name__}: {e}"[:500]}
+                    col[key] = {"error": f"{type(e).__name__}: {e}"[:2000]}   # ends with the trainer's log
         if rank == 0 and world == 1 and not args.no_cpu_baseline:
             out["cpu_baseline"] = cpu_baseline(sample_batch=16, steps=3, warmup=1)
 

@@ -28,6 +28,7 @@ import contextlib
 import ctypes as C
 import json
 import os
+import signal
 import sys
 import tempfile
 import time
@@ -66,7 +67,10 @@ def _seeded_state(arch):
 
 # ----------------------------------------------------------------------------------------------------- trainer
 def trainer_main(a):
+    import faulthandler
+
     import torch
+    faulthandler.register(signal.SIGUSR1)                # a server that waits in vain asks where the trainer stands
     from . import torch_col as tc
     from ._lib import SrtError, call
     from .step import ResNetStep
@@ -241,16 +245,20 @@ def _run(cleanup, duration_s, rate, policy, idle_ms, batch, seed, sm_partition, 
         return launcher not in _CHILDREN
 
     def wait_adjust_done(cid, limit_s=30):
-        """A trainer that has exited never answers: say so, with the end of its log, instead of waiting the limit out."""
+        """A trainer that has exited never answers: say so, with the end of its log, instead of waiting the limit out. One
+        that still runs leaves its Python stacks in the log first."""
         t1 = time.time()
         while True:
             try:
                 return ctl.wait_colocate_adjust_done(0, cid, 1000)
             except _lib.SrtError as e:
-                if trainer_exited():
-                    raise RuntimeError(f"{e}; the training process has exited: {_log_tail(log_path)}") from e
-                if time.time() - t1 > limit_s:
-                    raise
+                if not trainer_exited():
+                    if time.time() - t1 <= limit_s:
+                        continue
+                    os.kill(launcher.pid, signal.SIGUSR1)
+                    time.sleep(1.0)
+                raise RuntimeError(f"{e} (asked for {limit_s} s); the training process "
+                                   f"{'has exited' if trainer_exited() else 'still runs'}: {_log_tail(log_path)}") from e
 
     t0 = time.time()
     while not os.path.exists(result + ".ready"):

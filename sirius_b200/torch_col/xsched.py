@@ -18,7 +18,7 @@ def unregister_all_streams(): _streams.clear()
 
 
 def get_xqueue_size(stream=None) -> int:
-    return 0  # launches already handed to CUDA cannot be dropped; the executor never queues more than 8 units
+    return 0  # launches already handed to CUDA cannot be dropped; a training pass never queues more than 8 units
 
 
 def set_reject_cuda_calls(reject: bool):
